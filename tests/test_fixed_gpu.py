@@ -1,0 +1,84 @@
+"""Eigenvalues in 64-bit fixed point (the default path of the plain entry points).
+
+Every launch shape of the dispatch does the same arithmetic on a matrix, so a batch must give
+bitwise what its slices give in other shapes; parity with LAPACK at the edges of the order
+classes; graded and triangular matrices are left to the FP64 kernels, bitwise.
+"""
+import numpy as np
+import pytest
+
+from oracle import lapack_oracle as lo
+from tokura_zgeev_batched_gb300 import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+
+def solve(A, handle=None):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    w, f = api.zgeev_batched(A, handle=handle)
+    torch.cuda.synchronize()
+    return w.cpu().numpy(), f.cpu().numpy()
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 8, 9, 16, 17, 24, 25, 32, 33, 48, 49, 63, 64])
+def test_parity_at_class_edges(cuda, n):
+    import torch
+
+    for cls in ("gaussian", "vdv", "companion"):
+        A = wl.GENERATORS[cls](65, n, seed=5000 + n)
+        w, f = solve(torch.from_numpy(A).cuda())
+        rep = lo.parity_report(A, w, f)
+        assert rep["flag_mismatch"] == 0 and (f == 0).all(), (cls, rep)
+        if rep["well_conditioned"]:
+            assert rep["max_rel_err_well"] <= lo.TOL_REL_FRO, (cls, rep["max_rel_err_well"])
+
+
+@pytest.mark.parametrize("n,batches", [(4, (9000, 40000, 60001)), (7, (4000, 12000, 30001)), (13, (2000, 9000, 12001)),
+                                       (21, (1100, 4000, 6001)), (30, (1100, 4001)), (40, (700, 1500, 4001)),
+                                       (48, (900, 4001)), (61, (800, 1001, 4001))])
+def test_every_launch_shape_gives_the_same_bits(cuda, n, batches):
+    A = wl.torch_gaussian(max(batches), n, seed=5100 + n)
+    few = [solve(A[k:k + 5])[0] for k in (0, 3)]
+    for batch in batches:
+        w, f = solve(A[:batch])
+        assert (f == 0).all()
+        assert np.array_equal(w[:5].view(np.uint64), few[0].view(np.uint64)), batch
+        assert np.array_equal(w[3:8].view(np.uint64), few[1].view(np.uint64)), batch
+        tail = solve(A[batch - 6:batch])[0]
+        assert np.array_equal(w[-6:].view(np.uint64), tail.view(np.uint64)), batch
+
+
+@pytest.mark.parametrize("n", [3, 8, 20, 50])
+def test_graded_and_triangular_matrices_are_left_to_fp64(cuda, n):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A = wl.gaussian(12, n, seed=5200 + n)
+    d = 2.0 ** np.linspace(0, -40, n)
+    A[1] *= d[:, None] * d[None, :]  # graded rows and columns
+    A[4] = np.triu(A[4])
+    A[7] *= d[:, None]
+    A[9] = np.diag(d)
+    At = torch.from_numpy(A).cuda()
+    w, f = solve(At)
+    h = api.Handle()
+    assert h.set_shift_hints(0) == 0  # the FP64 iteration without hints
+    w64, f64 = solve(At, h)
+    left = [1, 4, 7, 9]
+    assert np.array_equal(w[left].view(np.uint64), w64[left].view(np.uint64))
+    assert np.array_equal(f, f64)
+    assert np.array_equal(np.sort(w[9].real), np.sort(d))
+
+
+def test_extreme_scales_and_exact_rows(cuda):
+    """The exponent of a matrix may be anything; eigenvalues scale with it exactly."""
+    import torch
+
+    A = wl.gaussian(8, 19, seed=5300)
+    w, _ = solve(torch.from_numpy(A).cuda())
+    for e in (-900, -300, 300, 900):
+        ws, f = solve(torch.from_numpy(np.ldexp(A.view(np.float64), e).view(np.complex128)).cuda())
+        assert (f == 0).all()
+        assert np.array_equal(np.ldexp(ws.view(np.float64), -e), w.view(np.float64))

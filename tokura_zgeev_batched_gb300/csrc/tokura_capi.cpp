@@ -283,5 +283,6 @@ extern "C" int tokuraSetShiftHints(tokurablas_t* handle, int mode) {
   if (handle == nullptr) return -1;
   if (mode < 0 || mode > 2) return -2;
   handle->shift_hints = mode;
+  handle->shift_hints_set = true;
   return 0;
 }

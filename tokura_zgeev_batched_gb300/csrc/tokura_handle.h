@@ -43,6 +43,7 @@ struct tokurablas_t {
   int balance_mode = 0;  // balancing before the eigenvalue solves: 0 none (the reference's behaviour) .. 3 both
   int ragged_hint_min_n = 48;  // mode 1: ragged matrices of this order and above get hints (65: none)
   int scaled_min_n = kScaledRotationDefaultMinN;  // plain QR with scaled rotations from this order (65: never)
+  bool shift_hints_set = false;  // tokuraSetShiftHints was called
   int shift_hints = 1;   // FP32 eigenvalue estimates as first shifts: 0 off, 1 uniform batches with
                          // n >= kShiftHintMinN, 2 every eigenvalue entry point and order (ragged too)
   tzg::HostPipeline pipe;  // host-buffer entry point state (guarded by pipe_mutex)
@@ -84,8 +85,17 @@ inline bool plain_lanes_valid(int lanes, bool allow_zero) {
          lanes == 32;
 }
 
+// Whether a call of order n starts in 64-bit fixed point (zgeev_fixed.cuh): with the default options. A launch
+// shape, rotation kind, shift strategy (any call of tokuraSetShiftHints: with hints the workspace holds the
+// estimates afterwards) or balancing set on the handle names a variant of the FP64 iteration, which then runs alone.
+inline bool use_fixed(const tokurablas_t* h, int n) {
+  return n > 1 && h->plain[n].lanes == 0 && h->plain_qr_lanes[n] == 0 &&
+         h->scaled_min_n == kScaledRotationDefaultMinN && !h->shift_hints_set && h->balance_mode == 0;
+}
+
 inline PlainConfig plain_config_for(const tokurablas_t* h, int n, int batch) {
   PlainConfig c = h->plain[n];
+  if (use_fixed(h, n)) c.fixed = h->sm_count;
   if (c.lanes == 0) {
     // Batches below a quarter of the lanes that fill the GPU spread each matrix
     // over more lanes, up to n/2 (two elements of a row or column per lane) and 32:

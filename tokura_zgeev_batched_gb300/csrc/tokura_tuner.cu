@@ -123,6 +123,18 @@ extern "C" TOKURA_API int tokuraAutotune(tokurablas_t* handle, int n_min, int n_
         }
       }
     }
+    // The default, which may start in fixed point (an order without a shape of its own takes it).
+    handle->plain[n] = PlainConfig{0, 0};
+    const PlainConfig chosen = plain_config_for(handle, n, batch_count);
+    if (chosen.fixed != 0) {
+      cudaError_t err;
+      const float ms = time_launches(stream, 2, [&]() {
+        return launch_plain(chosen, n, batch_count, A, eig, work, flag, default_itmax(n), stream, 0,
+                            use_shift_hints(handle, n), &handle->fj);
+      }, &err);
+      if (err != cudaSuccess) return 1;
+      if (ms < best) continue;
+    }
     handle->plain[n] = best_cfg;
   }
   return cudaStreamSynchronize(stream) == cudaSuccess ? 0 : 1;

@@ -1,0 +1,338 @@
+// Eigenvalues of upper Hessenberg matrices in 64-bit fixed point (zgeev_fixed.cuh).
+//
+// A group of L lanes of a warp owns a matrix, which stays in shared memory
+// (packed upper Hessenberg, real subdiagonals) from the first sweep to the
+// last. A sweep is one explicitly shifted QR step on the active window
+// [lo, hi], H - sigma I = Q R, H' = R Q + sigma I, with rotations
+// [conj(c) s; -s c], s real, so that subdiagonals stay real. Lane r holds the
+// indices j = lo + r, lo + r + L, ...: until rotation j is known index j is
+// column j, which receives rotation k of the rows (k, k+1) in step k and
+// carries its entry of row k+1 in registers; from step j + 1 on it is row j,
+// which receives rotation k-2 of the columns (k-2, k-1) in step k and carries
+// its entry of column k-1. So every index of the window does one complex
+// rotation in each of the window's steps, whether it is still a column or
+// already a row, each entry is loaded and stored once per half sweep, and the
+// only chain is rotation -> next column's entry -> next rotation. After the
+// window's last row, rotation hi is the phase that makes R(hi, hi) real.
+//
+// Matrices of one warp run their sweeps in lockstep; a matrix that is done, or whose
+// window is shorter, has its lanes idle until the others' step count is reached.
+#pragma once
+
+#include "zgeev_fixed.cuh"
+#include "zgeev_internal.h"
+#include "zgeev_lane.cuh"
+
+namespace tzg {
+
+// Per-matrix state between the kernels: a power-of-two exponent, or one of these.
+constexpr int kStateGeneral = -2147483647;  // left to the FP64 kernels (kStateDone: nothing left to do)
+
+// Entries of 16 bytes between consecutive matrices of a warp in shared memory: lanes of a quarter
+// warp reading consecutive entries of their own matrices then use different banks.
+template <int L>
+__host__ __device__ constexpr int fixed_stride(int count) {
+  return L >= 8 ? count : (count + 7 - ((count + 7 - L) & 7));
+}
+// Words of 16 bytes that a matrix uses beside its entries: the current rotation as columns take it ({c.re, s},
+// {-c.im, c.im}), the last four as rows do ({c.re, s}, {c.im, -c.im}), the next column's entry, and the
+// subdiagonals of the sweep's start.
+__host__ __device__ constexpr int qr_words(int n) { return 2 + 8 + 1 + (n + 1) / 2; }
+// A matrix has one entry in front (row lo of column lo - 1 for lo = 0) and one behind (row n of
+// column n - 1) its packed form; lanes without work in a step may read, not write, up to qr_slack
+// entries further.
+__host__ __device__ constexpr int qr_slack(int n) { return n + 8; }
+template <int L>
+__host__ __device__ constexpr int qr_stride(int n) {
+  return fixed_stride<L>(hess_count(n) + 2);
+}
+
+// kGlobal: the matrices stay in the workspace (in cache) instead of shared memory.
+template <int L, bool kGlobal>
+inline size_t fixed_qr_shared(int n) {
+  return ((size_t)(32 / L) * ((kGlobal ? 0 : qr_stride<L>(n)) + qr_words(n)) + (kGlobal ? 0 : qr_slack(n))) * 16;
+}
+
+// w 2^e rounded to nearest, with integer instructions unless the result is outside the normal range.
+__device__ __forceinline__ double fixed_to_double(long long w, int e) {
+  const unsigned long long m = w < 0 ? 0ull - (unsigned long long)w : (unsigned long long)w;
+  if (m == 0) return 0.0;
+  const int z = clz64(m), ex = e + 63 - z + 1023;
+  const unsigned long long sign = w < 0 ? 1ull << 63 : 0ull;
+  if (ex < 1 || ex > 2045) {
+    const int f = e + 62, a = f / 2, b = f - a;
+    return (double)w * 2.168404344971009e-19 * pow2(a) * pow2(b);  // 2^-62
+  }
+  const unsigned long long r = ((m << z) >> 10) + 1 >> 1;  // 2^52 .. 2^53
+  return __longlong_as_double((long long)(sign | (((unsigned long long)(ex - 1) << 52) + r)));
+}
+
+// Everything a lane keeps during a sweep. What bounds it: the 32x32-bit multiplier, one warp
+// instruction in four clocks of a sub-partition (a rotation is 36 of them, its coefficients 22), 60 % busy
+// at n = 16 (65,536 matrices, 9 warps per SM) and 50 % at n = 64 in shared memory (5.4 warps per SM); the rest is
+// the chain of a step with few warps to hide it. Making rotation k + 1 beside step k's work (18 more
+// multiplications) was 8 % faster at n >= 32 with the matrices in shared memory, 15-25 % slower below.
+template <int L, int T>
+struct QrLane {
+  cfx* H;          // packed matrix
+  int4* cur;       // current rotation for columns; then the ring of rows' rotations
+  cfx* next;       // entry (k, k) that rotation k is made from (L > 1)
+  long long* sub;  // subdiagonals of the window
+  Starts starts;
+  int rank, lo, m;
+  cfx carry[T];  // this lane's entries in flight, one per index
+  cfx ld[T];     // entries that the next step takes in
+  int at[T];     // and where they come from
+
+  // The steps of one sweep, `U` indices per lane in use.
+  template <int U>
+  __device__ __forceinline__ void sweep(int last) {
+    for (int kk = 0; kk <= last; ++kk) {
+      const int k = lo + kk;
+      __syncwarp();
+      cfx x = carry[0];
+      if (L > 1) {
+        x = *next;
+      } else {
+#pragma unroll
+        for (int t = 1; t < U; ++t)
+          if (kk == t) x = carry[t];
+      }
+      const long long y = kk < m ? sub[kk] : kZero;
+      {
+        const RotC g = make_rotc(x.x - kZero, x.y - kZero, y - kZero);
+        if (rank == 0) {
+          const int4 a = make_int4(g.cr.h, g.cr.l, g.s.h, g.s.l);
+          int4* const r = cur + 2 + (kk & 3) * 2;
+          cur[0] = a;
+          cur[1] = make_int4(-g.ci.h, -g.ci.l, g.ci.h, g.ci.l);
+          r[0] = a;
+          r[1] = make_int4(g.ci.h, g.ci.l, -g.ci.h, -g.ci.l);
+        }
+      }
+      __syncwarp();
+      const int4* const row = cur + 2 + ((kk - 2) & 3) * 2;
+      int4 ca[U], cb[U];
+#pragma unroll
+      for (int t = 0; t < U; ++t) {
+        const int4* const c = rank + t * L >= kk ? cur : row;
+        ca[t] = c[0];
+        cb[t] = c[1];
+      }
+      cfx o[U];
+#pragma unroll
+      for (int t = 0; t < U; ++t) {
+        const int4 a = ca[t], b = cb[t];
+        rotate(starts, Limbs{a.x, a.y}, Limbs{b.x, b.y}, Limbs{b.z, b.w}, Limbs{a.z, a.w}, Limbs{-a.z, -a.w}, carry[t],
+               ld[t], o[t], carry[t]);
+      }
+      const bool on = kk <= m + 1;
+#pragma unroll
+      for (int t = 0; t < U; ++t) {
+        const int i = rank + t * L;
+        if (on && i < m) H[at[t] - (i >= kk ? 1 : k)] = o[t];
+        if (kk <= m) at[t] += i > kk ? 1 : i == kk ? -1 : k + 1;
+        if (L > 1 && i == kk + 1) *next = carry[t];
+        ld[t] = H[at[t]];
+      }
+    }
+  }
+
+  __device__ __forceinline__ void run(int last, int used) {
+    if constexpr (T == 1) {
+      sweep<1>(last);
+    } else if constexpr (T == 2) {
+      if (used <= 1)
+        sweep<1>(last);
+      else
+        sweep<2>(last);
+    } else if constexpr (T == 4) {
+      if (used <= 1)
+        sweep<1>(last);
+      else if (used == 2)
+        sweep<2>(last);
+      else if (used == 3)
+        sweep<3>(last);
+      else
+        sweep<4>(last);
+    } else {
+      if (used <= 2)
+        sweep<2>(last);
+      else if (used <= 4)
+        sweep<4>(last);
+      else
+        sweep<T>(last);
+    }
+  }
+};
+
+template <int L, int T, bool kGlobal, class Batch>
+__global__ void __launch_bounds__(32) fixed_qr_kernel(int n, int batch, Batch B, cfx* __restrict__ hess,
+                                                       char* __restrict__ flag, int itmax, int* __restrict__ state,
+                                                       int one) {
+  constexpr int TW = 32 / L;
+  constexpr unsigned kAll = 0xffffffffu;
+  extern __shared__ __align__(16) char fixed_smem[];
+  const int lane = threadIdx.x & 31, rank = lane & (L - 1), slot = lane / L, base = lane & ~(L - 1);
+  const int count = hess_count(n), stride = qr_stride<L>(n);
+  // A block takes every gridDim-th group of matrices.
+  for (long long j0 = (long long)blockIdx.x * TW; j0 < batch; j0 += (long long)gridDim.x * TW) {
+  const long long j = j0 + slot;
+  // Whole warps stay together; lanes without a matrix keep an empty window.
+  const int st = j < batch ? state[j] : kStateDone;
+  const bool have = st != kStateDone && st != kStateGeneral;
+  if (!__any_sync(kAll, have)) continue;
+  cfx* H;
+  cfx* words = reinterpret_cast<cfx*>(fixed_smem);
+  if (kGlobal) {
+    H = hess + min(j, (long long)batch - 1) * hess_stride(n) + 1;
+  } else {
+    cfx* const sm = words + 1;
+    const int all = (int)min((long long)TW, batch - j0) * count;
+    for (int e = lane; e < all; e += 32) {
+      const int t = TW == 1 ? 0 : e / count;
+      sm[t * stride + (e - t * count)] = hess[(j0 + t) * hess_stride(n) + hess_lead(n) + (e - t * count)];
+    }
+    H = sm + slot * stride;
+    words += TW * stride;
+  }
+  words += slot * qr_words(n);
+  QrLane<L, T> Q;
+  Q.H = H;
+  Q.cur = reinterpret_cast<int4*>(words);
+  Q.next = words + 10;
+  Q.sub = reinterpret_cast<long long*>(words + 11);
+  Q.starts = make_starts(one);
+  Q.rank = rank;
+  if (rank == 0) H[count] = cfx{kZero, kZero};  // row n of the last column
+  __syncwarp();
+
+  int hi = have ? n - 1 : -1;
+  int its = 0, kdefl = 0, status = kConverged;
+#ifdef TOKURA_DEBUG_BOUNDS
+  int sweeps = 0;
+#endif
+  while (true) {
+    // Deflation: one scan of the subdiagonals gives the window.
+    int lo = 0;
+    unsigned long long small = 0;
+    const int top = __reduce_max_sync(kAll, hi);
+    if (top < 0) break;
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      if (t * L > top) break;
+      const int k = rank + t * L;
+      bool neg = false;
+      if (k >= 1 && k <= hi) {
+        const long long y = H[hess_idx(k, k - 1)].x - kZero;
+        const cfx d1 = H[hess_idx(k - 1, k - 1)], d2 = H[hess_idx(k, k)], up = H[hess_idx(k - 1, k)];
+        const long long yu = k >= 2 ? H[hess_idx(k - 1, k - 2)].x - kZero : 0;
+        const long long yd = k < hi ? H[hess_idx(k + 1, k)].x - kZero : 0;
+        neg = fixed_negligible(y, cfx{d1.x - kZero, d1.y - kZero}, cfx{d2.x - kZero, d2.y - kZero},
+                               cfx{up.x - kZero, up.y - kZero}, yu, yd);
+      }
+      if (L == 1) {
+        small |= (unsigned long long)neg << k;
+      } else {
+        const unsigned vote = (__ballot_sync(kAll, neg) >> base) & (L == 32 ? kAll : (1u << (L & 31)) - 1u);
+        small |= (unsigned long long)vote << (t * L);
+      }
+    }
+    while (hi >= 0) {
+      const unsigned long long below = small & ((2ull << hi) - 1ull);
+      lo = below ? 63 - clz64(below) : 0;
+      if (lo < hi) break;
+      // Converged: row hi becomes the (zero) row under the next window.
+      if (rank == 0) H[hess_idx(hi, hi - 1)] = cfx{kZero, kZero};
+      --hi;
+      its = 0;
+      kdefl = 0;
+    }
+    if (hi >= 0 && its > itmax) {
+      status = kNotConverged;
+      hi = -1;
+    }
+    const int m = hi < 0 ? -2 : hi - lo + 1;
+    const int steps = __reduce_max_sync(kAll, m + 2);
+    if (steps == 0) continue;
+    ++its;
+    ++kdefl;
+#ifdef TOKURA_DEBUG_BOUNDS
+    if (m > 0) ++sweeps;
+#endif
+    cfx sigma = {0, 0};
+    if (m > 0) {
+      const cfx d = H[hess_idx(hi, hi)];
+      if (kdefl % kExceptionalPeriod == 0) {  // ad hoc, towards zero: no larger than the matrix's norm
+        const bool bottom = kdefl % (2 * kExceptionalPeriod) == 0;
+        const cfx f = bottom ? d : H[hess_idx(lo, lo)];
+        const long long y = H[bottom ? hess_idx(hi, hi - 1) : hess_idx(lo + 1, lo)].x - kZero;
+        const long long h = mag64(y) - (mag64(y) >> 2);
+        sigma.x = f.x - kZero;
+        sigma.x += sigma.x < 0 ? h : -h;
+        sigma.y = f.y - kZero;
+      } else {
+        const cfx b = H[hess_idx(hi - 1, hi)];
+        const cfx e = wilkinson_correction(H[hess_idx(hi - 1, hi - 1)], cfx{b.x - kZero, b.y - kZero},
+                                           H[hess_idx(hi, hi - 1)].x - kZero, d);
+        sigma.x = d.x - kZero + e.x;
+        sigma.y = d.y - kZero + e.y;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < T; ++t) {  // H - sigma I
+      const int jj = min(lo + rank + t * L, n - 1);
+      if (rank + t * L < m) {
+        cfx* const d = H + hess_idx(jj, jj);
+        d->x -= sigma.x;
+        d->y -= sigma.y;
+      }
+      Q.at[t] = hess_idx(lo, jj) + 1;
+      Q.carry[t] = H[hess_idx(lo, jj)];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const int i = rank + t * L, jj = lo + i;
+      Q.ld[t] = H[Q.at[t]];
+      if (i < m) Q.sub[i] = H[hess_idx(jj + 1, jj)].x;
+    }
+    if (rank == 0) {
+      *Q.next = Q.carry[0];
+      Q.cur[2 + 6] = make_int4(1 << 30, 0, 0, 0);  // rotation lo - 1: none
+      Q.cur[2 + 7] = make_int4(0, 0, 0, 0);
+    }
+    Q.lo = lo;
+    Q.m = m;
+    const int used = (steps - 2 + L - 1) / L;
+    Q.run(steps - 1, used);
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const int jj = lo + rank + t * L;
+      if (rank + t * L < m) {
+        cfx* const d = H + hess_idx(jj, jj);
+        d->x += sigma.x;
+        d->y += sigma.y;
+      }
+    }
+    // Row lo's index also wrote beside the window; a split stays one whatever becomes of its neighbours.
+    if (m > 0 && rank == 0) H[hess_idx(lo, lo - 1)] = cfx{kZero, kZero};
+    __syncwarp();
+  }
+  if (have) {
+    for (int i = rank; i < n; i += L) {
+      const cfx d = H[hess_idx(i, i)];
+      put_ev(B.out(j, n) + i, make_double2(fixed_to_double(d.x - kZero, st), fixed_to_double(d.y - kZero, st)));
+    }
+    if (rank == 0) flag[j] = (char)status;
+  }
+#ifdef TOKURA_DEBUG_BOUNDS
+  if (have && rank == 0) dbg_record_sweeps(j, sweeps);
+#endif
+  __syncwarp();
+  }
+}
+
+}  // namespace tzg

@@ -16,6 +16,7 @@ struct PlainConfig {
   int scaled = 0;       // QR with scaled rotations (orders >= 7; zgeev_scaled_qr.cuh)
   int qr_lanes = 0;     // lanes per matrix of the QR phase when it is its own launch (shift hints); 0: `lanes`
   int scaled_qr = 0;    // `scaled` for the QR phase at qr_lanes
+  int fixed = 0;        // SMs of the device if the call starts in 64-bit fixed point (zgeev_fixed.cuh), else 0
 };
 
 // Iteration cap per eigenvalue: LAPACK's rule 30*max(10, n) unless overridden.

@@ -84,7 +84,9 @@ extern "C" TOKURA_API int tokura_zgeev_batched_gpu_noalloc(tokurablas_t* handle,
   if (cudaGetDevice(&dev) != cudaSuccess || dev != handle->device) return 1;
   double2* scratch = nullptr;
   if (tzg::noalloc_scratch_ptr(&scratch) != cudaSuccess) return 1;
-  const tzg::PlainConfig cfg = tzg::plain_config_for(handle, n, batch_count);
+  tzg::PlainConfig cfg = tzg::plain_config_for(handle, n, batch_count);
+  // The fixed-point kernels keep four bytes per matrix behind the staging area.
+  if (need + sizeof(int) * (size_t)batch_count > tzg::kNoAllocScratchBytes) cfg.fixed = 0;
   const int itmax = handle->itmax_override > 0 ? handle->itmax_override : tzg::default_itmax(n);
   const cudaError_t err =
       tzg::launch_plain(cfg, n, batch_count, reinterpret_cast<const double2*>(A),
