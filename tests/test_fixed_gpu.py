@@ -82,3 +82,30 @@ def test_extreme_scales_and_exact_rows(cuda):
         ws, f = solve(torch.from_numpy(np.ldexp(A.view(np.float64), e).view(np.complex128)).cuda())
         assert (f == 0).all()
         assert np.array_equal(np.ldexp(ws.view(np.float64), -e), w.view(np.float64))
+
+
+@pytest.mark.parametrize("batch,lo_n,hi_n", [(40, 1, 64), (700, 1, 64), (2500, 1, 33), (6000, 1, 17)])
+def test_ragged_gives_the_bits_of_the_uniform_calls(cuda, batch, lo_n, hi_n):
+    """Few and many matrices (both sets of launch shapes), every order, a graded one among them."""
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    ns = wl.ragged_sizes(batch, lo_n, hi_n, seed=5400 + batch)
+    mats = [wl.gaussian(1, int(n), seed=5500 + k)[0] for k, n in enumerate(ns)]
+    d = 2.0 ** np.linspace(0, -40, int(ns[5]))
+    mats[5] = mats[5] * d[:, None]
+    buf, n32, offs, eoffs = wl.pack_ragged(mats)
+    w, f = api.zgeev_ragged(torch.from_numpy(buf).cuda(), torch.from_numpy(n32))
+    w, f = w.cpu().numpy(), f.cpu().numpy()
+    assert (f == 0).all()
+    for n in np.unique(ns):
+        at = [k for k in np.nonzero(ns == n)[0] if k != 5]
+        if not at:
+            continue
+        wu, fu = solve(torch.from_numpy(np.stack([mats[k] for k in at])).cuda())
+        got = np.stack([w[eoffs[k]:eoffs[k] + n] for k in at])
+        assert np.array_equal(got.view(np.uint64), wu.view(np.uint64)), n
+    n = int(ns[5])
+    ref = lo.zgeev(mats[5][None])[0]
+    err = lo.matched_abs_errors(w[eoffs[5]:eoffs[5] + n][None], ref).max()
+    assert err <= lo.TOL_REL_FRO * np.linalg.norm(mats[5])

@@ -155,7 +155,8 @@ extern "C" int tokura_zgeev_ragged_gpu(tokurablas_t* handle, int batch_count, co
                                              total_elements, reinterpret_cast<const double2*>(A),
                                              reinterpret_cast<double2*>(eigenvalues), work, flag,
                                              handle->itmax_override, stream, handle->balance_mode,
-                                             tzg::ragged_hint_min_order(handle), &handle->fj, handle->scaled_min_n);
+                                             tzg::ragged_hint_min_order(handle), &handle->fj, handle->scaled_min_n,
+                                             tzg::use_fixed_ragged(handle));
   return err == cudaSuccess ? 0 : 1;
 }
 

@@ -28,7 +28,10 @@ struct HostPipeline {
 namespace tzg {
 // Default smallest order of the plain QR with scaled rotations.
 constexpr int kScaledRotationDefaultMinN = 16;
+// Default smallest order of the ragged shift hints.
+constexpr int kRaggedHintDefaultMinN = 48;
 }  // namespace tzg
+using tzg::kRaggedHintDefaultMinN;
 using tzg::kScaledRotationDefaultMinN;
 
 struct tokurablas_t {
@@ -41,7 +44,7 @@ struct tokurablas_t {
   tzg::PlainConfig real[65] = {};  // the same for the real (dgeev/sgeev) kernel
   int ragged_lanes = 0;  // lanes per matrix of the ragged solvers; 0 = chosen per launch
   int balance_mode = 0;  // balancing before the eigenvalue solves: 0 none (the reference's behaviour) .. 3 both
-  int ragged_hint_min_n = 48;  // mode 1: ragged matrices of this order and above get hints (65: none)
+  int ragged_hint_min_n = kRaggedHintDefaultMinN;  // mode 1: ragged matrices of this order and above get hints (65: none)
   int scaled_min_n = kScaledRotationDefaultMinN;  // plain QR with scaled rotations from this order (65: never)
   bool shift_hints_set = false;  // tokuraSetShiftHints was called
   int shift_hints = 1;   // FP32 eigenvalue estimates as first shifts: 0 off, 1 uniform batches with
@@ -90,6 +93,12 @@ inline bool plain_lanes_valid(int lanes, bool allow_zero) {
 // estimates afterwards) or balancing set on the handle names a variant of the FP64 iteration, which then runs alone.
 inline bool use_fixed(const tokurablas_t* h, int n) {
   return n > 1 && h->plain[n].lanes == 0 && h->plain_qr_lanes[n] == 0 &&
+         h->scaled_min_n == kScaledRotationDefaultMinN && !h->shift_hints_set && h->balance_mode == 0;
+}
+
+// The same for ragged calls.
+inline bool use_fixed_ragged(const tokurablas_t* h) {
+  return h->ragged_lanes == 0 && h->ragged_hint_min_n == kRaggedHintDefaultMinN &&
          h->scaled_min_n == kScaledRotationDefaultMinN && !h->shift_hints_set && h->balance_mode == 0;
 }
 

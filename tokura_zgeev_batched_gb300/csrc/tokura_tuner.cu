@@ -162,12 +162,14 @@ extern "C" TOKURA_API int tokuraAutotuneRagged(tokurablas_t* handle, int batch_c
   fill_sizes_kernel<<<1, 1, 0, stream>>>(n, off, batch_count, n_min, n_max, 0x5eed1234ULL);
   float best = 1e30f;
   int best_lanes = 0;
-  for (int lanes : {0, 1, 2, 4, 8}) {  // 0: lane width chosen per size bin
+  handle->ragged_lanes = 0;
+  const bool fixed = use_fixed_ragged(handle);
+  for (int lanes : {0, 1, 2, 4, 8}) {  // 0: the default (fixed point, or the lane width chosen per size bin)
     cudaError_t err;
     const float ms = time_launches(stream, 2, [&]() {
       return launch_ragged(lanes, handle->sm_count, batch_count, n, off, nullptr, total, A,
                            static_cast<double2*>(b.p[1]), b.p[2], static_cast<char*>(b.p[3]), 0, stream, 0,
-                           ragged_hint_min_order(handle), &handle->fj, handle->scaled_min_n);
+                           ragged_hint_min_order(handle), &handle->fj, handle->scaled_min_n, fixed && lanes == 0);
     }, &err);
     if (err != cudaSuccess) return 1;
     if (ms < best) {

@@ -258,21 +258,24 @@ __device__ __forceinline__ Reflector make_reflector(unsigned __int128 s, long lo
   return f;
 }
 
-template <int L, class Batch>
-__global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(int n, int batch, Batch B, cfx* __restrict__ hess,
+template <int L, class Work, class Batch>
+__global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, Batch B, cfx* __restrict__ hess,
                                                                      char* __restrict__ flag, int* __restrict__ state,
                                                                      int one) {
   constexpr int TW = L >= 32 ? 1 : 32 / L;
   extern __shared__ __align__(16) char fixed_smem[];
-  const int ld = n | 1, nn = n * n, stride = fixed_stride<(L > 8 ? 8 : L)>(n * ld + n);
   const int slot = L >= 32 ? 0 : (threadIdx.x & 31) / L;
-  const long long j = (long long)blockIdx.x * TW + slot;
+  FixedTile tile;
+  for (long long tix = blockIdx.x; work.tile(tix, TW, slot, tile); tix += gridDim.x) {
+  const int n = tile.n, ld = n | 1, nn = n * n, stride = fixed_stride<(L > 8 ? 8 : L)>(n * ld + n);
+  const long long j = tile.j;
+  const bool exists = slot < tile.count;
   cfx* const A = reinterpret_cast<cfx*>(fixed_smem) + slot * stride;
   int4* const U = reinterpret_cast<int4*>(A + n * ld);
   const FixedGroup<L> G(reinterpret_cast<unsigned long long*>(fixed_smem + (size_t)TW * stride * 16));
   const Starts k = make_starts(one);
   int st = kStateDone;  // this matrix's state; only exponents go on to the reduction
-  if (j < batch) {
+  if (exists) {
     if (!B.valid(j)) {
       const double nan = __longlong_as_double(0x7ff8000000000000LL);
       for (int i = G.rank; i < n; i += L) put_ev(B.out(j, n) + i, make_double2(nan, nan));
@@ -335,7 +338,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(int n, int 
     if (G.rank == 0) state[j] = st;
   }
   const bool have = st != kStateDone && st != kStateGeneral;
-  if (L > 32 ? !have : !__any_sync(0xffffffffu, have)) return;  // block- or warp-uniform
+  if (L > 32 ? !have : !__any_sync(0xffffffffu, have)) continue;  // block- or warp-uniform
   G.sync();
 
   for (int r = 0; r + 1 < n; ++r) {
@@ -390,9 +393,11 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(int n, int 
     G.sync();
   }
   if (have) {
-    cfx* const out = hess + j * hess_stride(n) + hess_lead(n);
+    cfx* const out = hess + tile.where + (long long)slot * hess_stride(n) + hess_lead(n);
     for (int c = 0; c < n; ++c)
       for (int r = G.rank; r <= min(c + 1, n - 1); r += L) out[hess_idx(r, c)] = A[c * ld + r];
+  }
+  G.sync();
   }
 }
 

@@ -166,32 +166,56 @@ struct QrLane {
   }
 };
 
-template <int L, int T, bool kGlobal, class Batch>
-__global__ void __launch_bounds__(32) fixed_qr_kernel(int n, int batch, Batch B, cfx* __restrict__ hess,
-                                                       char* __restrict__ flag, int itmax, int* __restrict__ state,
+// Some matrices of one order that a warp (or block) takes together.
+struct FixedTile {
+  int n, count;     // order, matrices (the slots 0 .. count - 1)
+  long long j;      // this slot's matrix
+  long long where;  // first entry of slot 0's packed form in the workspace (slots follow one another)
+};
+
+// Work of a uniform batch: matrices 0 .. batch - 1 in order, `tw` to a tile.
+struct UniformWork {
+  int n, batch;
+  __device__ __forceinline__ bool tile(long long t, int tw, int slot, FixedTile& out) const {
+    const long long j0 = t * tw;
+    if (j0 >= batch) return false;
+    out.n = n;
+    out.count = (int)min((long long)tw, batch - j0);
+    out.j = j0 + slot;
+    out.where = j0 * hess_stride(n);
+    return true;
+  }
+};
+
+// `itmax` 0: the default for each order.
+template <int L, int T, bool kGlobal, class Work, class Batch>
+__global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* __restrict__ hess,
+                                                       char* __restrict__ flag, int itmax0, int* __restrict__ state,
                                                        int one) {
   constexpr int TW = 32 / L;
   constexpr unsigned kAll = 0xffffffffu;
   extern __shared__ __align__(16) char fixed_smem[];
   const int lane = threadIdx.x & 31, rank = lane & (L - 1), slot = lane / L, base = lane & ~(L - 1);
-  const int count = hess_count(n), stride = qr_stride<L>(n);
-  // A block takes every gridDim-th group of matrices.
-  for (long long j0 = (long long)blockIdx.x * TW; j0 < batch; j0 += (long long)gridDim.x * TW) {
-  const long long j = j0 + slot;
+  // A block takes every gridDim-th tile.
+  FixedTile tile;
+  for (long long tix = blockIdx.x; work.tile(tix, TW, slot, tile); tix += gridDim.x) {
+  const int n = tile.n, count = hess_count(n), stride = qr_stride<L>(n);
+  const int itmax = itmax0 > 0 ? itmax0 : default_itmax(n);
+  const long long j = tile.j;
   // Whole warps stay together; lanes without a matrix keep an empty window.
-  const int st = j < batch ? state[j] : kStateDone;
+  const int st = slot < tile.count ? state[j] : kStateDone;
   const bool have = st != kStateDone && st != kStateGeneral;
   if (!__any_sync(kAll, have)) continue;
   cfx* H;
   cfx* words = reinterpret_cast<cfx*>(fixed_smem);
   if (kGlobal) {
-    H = hess + min(j, (long long)batch - 1) * hess_stride(n) + 1;
+    H = hess + tile.where + (long long)min(slot, tile.count - 1) * hess_stride(n) + 1;
   } else {
     cfx* const sm = words + 1;
-    const int all = (int)min((long long)TW, batch - j0) * count;
+    const int all = tile.count * count;
     for (int e = lane; e < all; e += 32) {
       const int t = TW == 1 ? 0 : e / count;
-      sm[t * stride + (e - t * count)] = hess[(j0 + t) * hess_stride(n) + hess_lead(n) + (e - t * count)];
+      sm[t * stride + (e - t * count)] = hess[tile.where + t * hess_stride(n) + hess_lead(n) + (e - t * count)];
     }
     H = sm + slot * stride;
     words += TW * stride;

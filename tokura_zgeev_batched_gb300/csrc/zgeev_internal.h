@@ -47,7 +47,8 @@ size_t ragged_workspace_bytes(int batch, long long total_elements);
 cudaError_t launch_ragged(int lanes, int sms, int batch, const int* n, const long long* offsets,
                           const long long* eig_offsets, long long total_elements, const double2* A, double2* eig,
                           void* work, char* flag, int itmax_override, cudaStream_t stream, int balance = 0,
-                          int hint_min_n = 0, const ForkJoin* fj = nullptr, int scaled_min_n = 65);  // per lane
+                          int hint_min_n = 0, const ForkJoin* fj = nullptr, int scaled_min_n = 65,  // per lane
+                          bool fixed = false);  // start in fixed point (zgeev_fixed.cuh)
 
 // Backward (Abar from A, eigenvalues and their gradients).
 size_t backward_workspace_bytes(int n, int batch);

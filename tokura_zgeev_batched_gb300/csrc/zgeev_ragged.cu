@@ -158,7 +158,8 @@ cudaError_t ragged_prepare(int lanes, int sms, int batch, const int* n, const lo
 cudaError_t launch_ragged(int lanes, int sms, int batch, const int* n, const long long* offsets,
                           const long long* eig_offsets, long long total_elements, const double2* A, double2* eig,
                           void* work, char* flag, int itmax_override, cudaStream_t stream, int balance,
-                          int hint_min_n, const ForkJoin* fj, int scaled_min_n) {
+                          int hint_min_n, const ForkJoin* fj, int scaled_min_n, bool fixed) {
+  if (fixed) hint_min_n = 0;
   // Shift hints for the matrices of order >= hint_min_n (0: none).
   const bool hints = hint_min_n > 0 && hint_min_n <= kMaxN;
   // lanes == 0: each size bin gets its own lane width from the planner (ragged_plan_kernel).
@@ -170,6 +171,7 @@ cudaError_t launch_ragged(int lanes, int sms, int batch, const int* n, const lon
   int* state = reinterpret_cast<int*>(w + lay.state_off);
   const bool split = hints && fj != nullptr && fj->aux != nullptr;
   std::unique_lock<std::mutex> lock;
+  if (fixed && fj != nullptr && fj->aux != nullptr) lock = std::unique_lock<std::mutex>(*fj->mu);
   cudaError_t err = cudaSuccess;
   if (split) {  // the estimator starts first, beside the planning and the prepare phase
     lock = std::unique_lock<std::mutex>(*fj->mu);
@@ -184,8 +186,12 @@ cudaError_t launch_ragged(int lanes, int sms, int batch, const int* n, const lon
   err = ragged_prepare(lanes, sms, batch, n, offsets, eig_offsets, total_elements, lay, work, flag, stream, &plan,
                        &sorted, &eo);
   if (err != cudaSuccess) return err;
-  const RaggedArgs args{offsets, eo, A, eig, nullptr, nullptr, nullptr, stage, total_elements, flag, sorted,
-                        itmax_override, balance, est, state, hint_min_n, scaled_min_n};
+  RaggedArgs args{offsets, eo, A, eig, nullptr, nullptr, nullptr, stage, total_elements, flag, sorted,
+                  itmax_override, balance, est, state, hint_min_n, fixed, scaled_min_n};
+  if (fixed) {
+    if ((err = ragged_launch_fixed(sms, batch, plan, args, stream, fj)) != cudaSuccess) return err;
+    return launch_ragged_kernel<false, false, kPhaseAll>(lanes, sms, plan, args, stream);
+  }
   if (split) return ragged_launch_phases(lanes, sms, plan, args, balance != 0, stream, *fj);
   if (balance != 0) return launch_ragged_kernel<false, true, kPhaseAll>(lanes, sms, plan, args, stream);
   return launch_ragged_kernel<false, false, kPhaseAll>(lanes, sms, plan, args, stream);

@@ -6,6 +6,7 @@
 
 #include "zgeev_backward.cuh"
 #include "zgeev_estimate.cuh"
+#include "zgeev_fixed_qr.cuh"
 #include "zgeev_internal.h"
 #include "zgeev_lane.cuh"
 #include "zgeev_scaled_qr.cuh"
@@ -89,6 +90,7 @@ struct RaggedArgs {
   const float2* est;     // forward: FP32 shift hints, kMaxN per matrix (or null)
   int* state;            // forward, split solve: pre-scaling exponent or kStateDone per matrix
   int est_min_n;         // forward: orders from which est holds hints
+  bool left_only = false;  // forward, after the fixed-point kernels: n = 1 and what they left (state)
   int scaled_min_n = 65;  // QR with scaled rotations from order max(7, lanes * scaled_min_n); > 64: never
 };
 
@@ -144,6 +146,7 @@ __device__ __forceinline__ void ragged_tile(const RaggedBin& bin, int t, const R
     status = backward_matrix<L>(a.A + a.offsets[j], a.lam + a.eoff[j], a.gbar + a.eoff[j], a.gA + a.offsets[j], V,
                                 G, itmax, scaled ? nb : kMaxN + 1);
   } else if (kPhase == kPhaseAll) {
+    if (a.left_only && nb > 1 && a.state[j] != kStateGeneral) return;  // group-uniform
     int shift;
     const MatView M{base, nb, tw};
     status = prepare_matrix<L, kBalance>(SrcContig{a.A + a.offsets[j]}, M, G, a.eig + a.eoff[j], a.balance, shift);
@@ -244,5 +247,9 @@ cudaError_t ragged_fork_estimates(int sms, int batch, const int* n, const long l
 // Prepare phase on `stream`, join with the estimator, QR phase (*fj.mu held).
 cudaError_t ragged_launch_phases(int lanes, int sms, RaggedPlan* plan, const RaggedArgs& args, bool balance,
                                  cudaStream_t stream, const ForkJoin& fj);
+
+// The forward in fixed point (zgeev_ragged_fixed.cu; *fj.mu held if there is a second stream).
+cudaError_t ragged_launch_fixed(int sms, int batch, RaggedPlan* plan, const RaggedArgs& args, cudaStream_t stream,
+                                const ForkJoin* fj);
 
 }  // namespace tzg

@@ -1,0 +1,101 @@
+// Ragged forward in 64-bit fixed point (zgeev_fixed.cuh): the planner's bins (matrices sorted by order) are
+// cut into classes of neighbouring orders, each with the launch shapes of a uniform batch of its largest order:
+//   caller's stream: [planning] --fork-- [orders 49..64, 33..48] --join-- [FP64: what was left]
+//   second stream:                 \---- [orders 25..32 .. 2..4] --/
+// The classes above n = 32 keep their matrices in the workspace and the others in shared memory, so the two
+// streams' kernels fit on an SM together, and one's last, half-empty wave is filled by the other.
+#include "zgeev_fixed_launch.cuh"
+#include "zgeev_ragged.cuh"
+
+namespace tzg {
+
+// Matrices of orders nhi down to nlo; a tile holds matrices of one order.
+struct RaggedWork {
+  const RaggedPlan* plan;
+  const int* sorted;
+  int nhi, nlo;
+  __device__ __forceinline__ bool tile(long long t, int tw, int slot, FixedTile& out) const {
+    if (plan->overflow) return false;
+    for (int nb = nhi; nb >= nlo; --nb) {
+      const RaggedBin& bin = plan->bins[kMaxN - nb];
+      const int tiles = (bin.count + tw - 1) / tw;
+      if (t < tiles) {
+        const int p = (int)t * tw;
+        out.n = nb;
+        out.count = min(tw, bin.count - p);
+        out.j = slot < out.count ? sorted[bin.first + p + slot] : 0;
+        out.where = bin.stage + (long long)p * hess_stride(nb);
+        return true;
+      }
+      t -= tiles;
+    }
+    return false;
+  }
+};
+
+struct RaggedBatch {
+  const double2* A;
+  const long long* offsets;
+  const long long* eoff;
+  double2* eig;
+  __device__ __forceinline__ bool valid(long long) const { return true; }
+  __device__ __forceinline__ SrcContig src(long long j) const { return SrcContig{A + offsets[j]}; }
+  __device__ __forceinline__ double2* out(long long j, int) const { return eig + eoff[j]; }
+};
+
+cudaError_t ragged_launch_fixed(int sms, int batch, RaggedPlan* plan, const RaggedArgs& args, cudaStream_t stream,
+                                const ForkJoin* fj) {
+  const RaggedBatch B{args.A, args.offsets, args.eoff, args.eig};
+  cfx* hess = reinterpret_cast<cfx*>(args.stage);
+  const int itmax = args.itmax_override;
+  const bool two = fj != nullptr && fj->aux != nullptr;
+  cudaError_t err = cudaSuccess;
+  cudaStream_t side = stream;
+  if (two) {
+    if ((err = cudaEventRecord(fj->fork, stream)) != cudaSuccess) return err;
+    if ((err = cudaStreamWaitEvent(fj->aux, fj->fork, 0)) != cudaSuccess) return err;
+    side = fj->aux;
+  }
+  const long long many = (long long)sms * 32;
+  auto fits = [&](int lanes, int warps) { return (long long)batch * lanes <= many * warps; };
+#define TZG_HESS(NHI, NLO, L, STREAM)                                                                       \
+  if (err == cudaSuccess)                                                                                   \
+    err = launch_fixed_hess<L>(RaggedWork{plan, args.sorted, NHI, NLO}, NHI, batch, B, hess, args.flag, args.state, \
+                               many, STREAM)
+#define TZG_QR(NHI, NLO, L, T, G, BLOCKS, STREAM)                                                             \
+  if (err == cudaSuccess)                                                                                     \
+    err = launch_fixed_qr<L, T, G>(RaggedWork{plan, args.sorted, NHI, NLO}, NHI, batch, B, hess, args.flag, itmax, \
+                                   args.state, BLOCKS, STREAM)
+  TZG_HESS(64, 49, 128, stream);
+  TZG_HESS(48, 33, 128, stream);
+  TZG_QR(64, 49, 32, 2, true, (long long)sms * 24, stream);
+  TZG_QR(48, 33, 32, 2, true, (long long)sms * 24, stream);
+  TZG_HESS(32, 25, 32, side);
+  TZG_HESS(24, 17, 32, side);
+  TZG_HESS(16, 9, 16, side);
+  TZG_HESS(8, 5, 8, side);
+  TZG_HESS(4, 2, 4, side);
+  if (fits(8, 16)) {  // few matrices: as the small uniform batches
+    TZG_QR(32, 25, 32, 1, false, many, side);
+    TZG_QR(24, 17, 32, 1, false, many, side);
+    TZG_QR(16, 9, 16, 1, false, many, side);
+    TZG_QR(8, 5, 8, 1, false, many, side);
+    TZG_QR(4, 2, 4, 1, false, many, side);
+  } else {
+    TZG_QR(32, 25, 16, 2, false, many, side);
+    TZG_QR(24, 17, 8, 4, false, many, side);
+    TZG_QR(16, 9, 4, 4, false, many, side);
+    TZG_QR(8, 5, 2, 4, false, many, side);
+    TZG_QR(4, 2, 1, 4, false, many, side);
+  }
+#undef TZG_HESS
+#undef TZG_QR
+  if (two) {  // also after a failed launch: the second stream rejoins the caller's
+    const cudaError_t e1 = cudaEventRecord(fj->join, fj->aux);
+    const cudaError_t e2 = cudaStreamWaitEvent(stream, fj->join, 0);
+    if (err == cudaSuccess) err = e1 != cudaSuccess ? e1 : e2;
+  }
+  return err;
+}
+
+}  // namespace tzg
