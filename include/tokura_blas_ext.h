@@ -95,6 +95,20 @@ TOKURA_API int tokuraGetPlainConfig(const tokurablas_t* handle, int n, int batch
  * Returns 0, -1 NULL handle, -2 n out of range, -3 bad lanes. */
 TOKURA_API int tokuraSetPlainQrLanes(tokurablas_t* handle, int n, int lanes_per_matrix);
 
+/* tokura_zgeev_batched_gpu on the FP64 kernels alone. The plain, layout,
+ * host-buffer, workspace-free and ragged eigenvalue calls and the eigenvector
+ * call start in 64-bit fixed point
+ * (csrc/zgeev_fixed.cuh: the matrix as 64-bit integers with one exponent,
+ * errors below the FP64 kernels' in norm; graded and triangular matrices are
+ * left to those) unless the handle has a launch shape, rotation kind, shift
+ * strategy or balancing set. The uniform gradient, whose results depend on the
+ * last bits of the forward where a spectrum is ill-conditioned, takes this
+ * call's eigenvalues in the torch binding. Arguments and return codes as
+ * tokura_zgeev_batched_gpu. */
+TOKURA_API int tokura_zgeev_batched_gpu_fp64(tokurablas_t* handle, int n, int batch_count, cuDoubleComplex* A,
+                                             cuDoubleComplex* eigenvalues, cuDoubleComplex* work, char* flag,
+                                             cudaStream_t cudastream);
+
 /* Autotuner (replaces the reference's build-time tuner,
  * src/TOKURA_ZHSEQR_BATCHED_GEHRD_TUNING_main.cu:89-227, and its generated
  * tables). For each order n in [n_min, n_max], times every plain-kernel shape

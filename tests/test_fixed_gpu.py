@@ -109,3 +109,51 @@ def test_ragged_gives_the_bits_of_the_uniform_calls(cuda, batch, lo_n, hi_n):
     ref = lo.zgeev(mats[5][None])[0]
     err = lo.matched_abs_errors(w[eoffs[5]:eoffs[5] + n][None], ref).max()
     assert err <= lo.TOL_REL_FRO * np.linalg.norm(mats[5])
+
+
+@pytest.mark.parametrize("n", [4, 5, 8, 9, 16, 17, 32, 33, 64])
+def test_eigenvectors_from_fixed_point_schur_forms(cuda, n):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    for k in (0, 1):
+        A = wl.vdv(37, n, seed=5700 + n) if k == 0 else wl.gaussian(37, n, seed=5700 + n)
+        A[3] = np.tril(A[3]) + np.diag(np.arange(n))
+        M = torch.from_numpy(A).cuda()
+        w, VL, VR, f = api.zgeev_vectors(M)
+        assert (f == 0).all()
+        fro = torch.linalg.norm(M, dim=(1, 2))[:, None, None]
+        assert float(((M @ VR - VR * w[:, None, :]).abs() / fro).max()) <= 1e-12 * n
+        assert float(((VL.mH @ M - w[:, :, None] * VL.mH).abs() / fro).max()) <= 1e-12 * n
+        assert torch.allclose(torch.linalg.norm(VR, dim=1), torch.ones_like(w.real), atol=1e-13)
+        rep = lo.parity_report(A, w.cpu().numpy(), f.cpu().numpy())
+        assert rep["max_rel_err_well"] <= lo.TOL_REL_FRO or not rep["well_conditioned"]
+    bad = M.clone()
+    bad[5, 1, 2] = complex("nan")
+    wb, VLb, VRb, fb = api.zgeev_vectors(bad)
+    keep = [k for k in range(37) if k != 5]
+    assert fb[5] == 2 and torch.isnan(wb[5].real).all() and torch.isnan(VRb[5].real).all()
+    assert torch.equal(torch.view_as_real(VRb[keep].contiguous()), torch.view_as_real(VR[keep].contiguous()))
+
+
+def test_schur_sweep_cap(cuda):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A = torch.from_numpy(wl.gaussian(20, 24, seed=5800)).cuda()
+    h = api.Handle()
+    assert h.set_sweep_cap(1) == 0
+    w, VL, VR, f = api.zgeev_vectors(A, handle=h)
+    assert (f == 1).all() and bool(torch.isfinite(torch.view_as_real(w)).all())
+
+
+def test_fp64_call_is_the_hinted_fp64_path(cuda):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A = torch.from_numpy(wl.gaussian(50, 20, seed=5900)).cuda()
+    w, f = api.zgeev_batched(A, fp64=True)
+    h = api.Handle()
+    assert h.set_shift_hints(1) == 0
+    w1, f1 = api.zgeev_batched(A, handle=h)
+    assert torch.equal(torch.view_as_real(w), torch.view_as_real(w1)) and (f == 0).all()

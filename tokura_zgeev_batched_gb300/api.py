@@ -31,6 +31,11 @@ _SIGNATURES = {
         [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
          ctypes.c_void_p, ctypes.c_void_p],
     ),
+    "tokura_zgeev_batched_gpu_fp64": (
+        ctypes.c_int,
+        [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+         ctypes.c_void_p, ctypes.c_void_p],
+    ),
     "tokuraSetSweepCap": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     "tokuraSetPlainConfig": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "tokuraSetPlainQrLanes": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int]),
@@ -277,12 +282,13 @@ def default_handle() -> Handle:
     return _DEFAULT_HANDLE
 
 
-def zgeev_batched(A, handle: Handle | None = None, work=None, stream=None):
+def zgeev_batched(A, handle: Handle | None = None, work=None, stream=None, fp64: bool = False):
     """Eigenvalues of a batch of square complex128 CUDA matrices ``A[..., n, n]``.
 
     Returns ``(eigenvalues[..., n], flag[...])`` (flag int8: 0 converged,
     1 iteration cap hit, 2 non-finite input). A is not modified. Runs on the
     current torch stream unless ``stream`` (a torch.cuda.Stream) is given.
+    ``fp64``: on the FP64 kernels alone (tokura_zgeev_batched_gpu_fp64).
     """
     import torch
 
@@ -305,8 +311,9 @@ def zgeev_batched(A, handle: Handle | None = None, work=None, stream=None):
         work = torch.empty(need, dtype=torch.uint8, device=A.device)
     s = stream if stream is not None else torch.cuda.current_stream(A.device)
     h = handle if handle is not None else default_handle()
-    status = tokura_zgeev_batched_gpu(h, n, batch, Ab.data_ptr(), eig.data_ptr(), work.data_ptr(), flag.data_ptr(),
-                                      s.cuda_stream)
+    call = lib().tokura_zgeev_batched_gpu_fp64 if fp64 else lib().tokura_zgeev_batched_gpu
+    status = int(call(_ptr(h), n, batch, Ab.data_ptr(), eig.data_ptr(), work.data_ptr(), flag.data_ptr(),
+                      s.cuda_stream))
     if status != 0:
         raise RuntimeError(f"tokura_zgeev_batched_gpu returned {status}")
     return eig.reshape(*batch_shape, n), flag.reshape(batch_shape)

@@ -18,7 +18,8 @@ from . import api
 class _EigvalsFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, A, handle):
-        eig, flag = api.zgeev_batched(A, handle=handle)
+        # The backward's FP64 Schur form starts from these eigenvalues.
+        eig, flag = api.zgeev_batched(A, handle=handle, fp64=True)
         ctx.save_for_backward(A, eig)
         ctx.handle = handle
         ctx.mark_non_differentiable(flag)

@@ -66,9 +66,8 @@ extern "C" size_t tokura_get_zgeeveigenvaluesgetworspacesize(int n, int batch_co
   return sizeof(cuDoubleComplex) * nn * (size_t)batch_count + sizeof(cuDoubleComplex) * (size_t)n * (size_t)batch_count;
 }
 
-extern "C" int tokura_zgeev_batched_gpu(tokurablas_t* handle, int n, int batch_count, cuDoubleComplex* A,
-                                        cuDoubleComplex* eigenvalues, cuDoubleComplex* work, char* flag,
-                                        cudaStream_t cudastream) {
+static int plain_call(tokurablas_t* handle, int n, int batch_count, cuDoubleComplex* A, cuDoubleComplex* eigenvalues,
+                      cuDoubleComplex* work, char* flag, cudaStream_t cudastream, bool fixed) {
   if (handle == nullptr) return -1;
   if (!(n > 0 && n <= TOKURA_ZGEEV_BATCHED_MAX_MATRIX_SIZE)) return -2;
   if (A == nullptr) return -3;
@@ -76,13 +75,26 @@ extern "C" int tokura_zgeev_batched_gpu(tokurablas_t* handle, int n, int batch_c
   if (work == nullptr) return -5;
   if (!(batch_count > 0)) return -6;
   if (flag == nullptr) return -7;
-  const PlainConfig cfg = tzg::plain_config_for(handle, n, batch_count);
+  PlainConfig cfg = tzg::plain_config_for(handle, n, batch_count);
+  if (!fixed) cfg.fixed = 0;
   const int itmax = handle->itmax_override > 0 ? handle->itmax_override : tzg::default_itmax(n);
   const cudaError_t err = tzg::launch_plain(cfg, n, batch_count, reinterpret_cast<const double2*>(A),
                                             reinterpret_cast<double2*>(eigenvalues),
                                             reinterpret_cast<double2*>(work), flag, itmax, cudastream,
                                             handle->balance_mode, tzg::use_shift_hints(handle, n), &handle->fj);
   return err == cudaSuccess ? 0 : 1;
+}
+
+extern "C" int tokura_zgeev_batched_gpu(tokurablas_t* handle, int n, int batch_count, cuDoubleComplex* A,
+                                        cuDoubleComplex* eigenvalues, cuDoubleComplex* work, char* flag,
+                                        cudaStream_t cudastream) {
+  return plain_call(handle, n, batch_count, A, eigenvalues, work, flag, cudastream, true);
+}
+
+extern "C" int tokura_zgeev_batched_gpu_fp64(tokurablas_t* handle, int n, int batch_count, cuDoubleComplex* A,
+                                             cuDoubleComplex* eigenvalues, cuDoubleComplex* work, char* flag,
+                                             cudaStream_t cudastream) {
+  return plain_call(handle, n, batch_count, A, eigenvalues, work, flag, cudastream, false);
 }
 
 extern "C" int tokuraSetSweepCap(tokurablas_t* handle, int cap) {
@@ -262,7 +274,8 @@ extern "C" int tokura_zgeev_vectors_batched_gpu(tokurablas_t* handle, int n, int
   const cudaError_t err = tzg::launch_vectors(
       lanes, n, batch_count, reinterpret_cast<const double2*>(A), reinterpret_cast<double2*>(eigenvalues),
       reinterpret_cast<double2*>(VL), reinterpret_cast<double2*>(VR), static_cast<double2*>(work), flag, itmax, stream,
-      tzg::use_shift_hints(handle, n), &handle->fj, tzg::scaled_threshold(handle, lanes));
+      tzg::use_shift_hints(handle, n), &handle->fj, tzg::scaled_threshold(handle, lanes),
+      tzg::use_fixed_schur(handle, n));
   return err == cudaSuccess ? 0 : 1;
 }
 

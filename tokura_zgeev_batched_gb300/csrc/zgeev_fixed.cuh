@@ -71,7 +71,7 @@ TZG_HD int high(long long v) { return (int)(v >> 32); }
 TZG_HD Limbs entry_limbs(long long s) {
   Limbs r;
   r.h = (int)(s >> 32);
-  r.l = (int)((unsigned)s + 0x80000000u);
+  r.l = (int)((unsigned)s ^ 0x80000000u);
   return r;
 }
 TZG_HD Limbs limbs(long long v) {
@@ -295,13 +295,13 @@ TZG_HD cfx wilkinson_correction(cfx a, cfx b, long long y, cfx d) {
 // Deflation test of the real subdiagonal y between diagonal entries d1
 // (above) and d2, with the entry `up` opposite it and its neighbouring
 // subdiagonals yu, yd: the Ahues-Tisseur criterion (LAPACK Working Note 122)
-// at 2^-52, or at most kFixedSmall. All V values.
-TZG_HD bool fixed_negligible(long long y, cfx d1, cfx d2, cfx up, long long yu, long long yd) {
+// at `ulps` times 2^-52, or at most kFixedSmall. All V values.
+TZG_HD bool fixed_negligible(long long y, cfx d1, cfx d2, cfx up, long long yu, long long yd, int ulps = 1) {
   const long long h = y < 0 ? -y : y;
   if (h <= kFixedSmall) return true;
   unsigned long long tst = mag64(d1.x) + mag64(d1.y) + mag64(d2.x) + mag64(d2.y);
   if (tst == 0) tst = mag64(yu) + mag64(yd);
-  if ((unsigned long long)h > (tst >> 52)) return false;
+  if ((unsigned long long)h > (tst >> 52) * ulps) return false;
   const float k32 = 2.3283064365386963e-10f;
   const float h1 = mulf(fx2f(h), k32), hu = mulf(abs1f(fx2f(up.x), fx2f(up.y)), k32);
   const float ab = fmaxf(h1, hu), ba = fminf(h1, hu);
@@ -309,7 +309,7 @@ TZG_HD bool fixed_negligible(long long y, cfx d1, cfx d2, cfx up, long long yu, 
   const float e2 = mulf(abs1f(fx2f(d2.x), fx2f(d2.y)), k32);
   const float aa = fmaxf(e2, dd), bb = fminf(e2, dd);
   const float s = addf(aa, ab);
-  const float ulp = 2.220446049250313e-16f;
+  const float ulp = mulf(2.220446049250313e-16f, (float)ulps);
   return mulf(ba, ab / s) <= fmaxf((float)kFixedSmall * k32, mulf(ulp, mulf(bb, aa / s)));
 }
 
@@ -320,5 +320,11 @@ TZG_HD int hess_count(int n) { return n < 2 ? n : hess_col(n - 1) + n; }
 // In the workspace, matrices follow one another; from n = 5 on each has an entry in front and one behind.
 TZG_HD int hess_lead(int n) { return n >= 5 ? 1 : 0; }
 TZG_HD int hess_stride(int n) { return hess_count(n) + 2 * hess_lead(n); }
+
+// Entries of a unitary matrix: kFixedOne is 1 (its columns' norms stay far below the entries' bound).
+constexpr int kFixedOneBits = 60;
+constexpr long long kFixedOne = 1LL << kFixedOneBits;
+// Where a Schur form's matrices are n^2 entries apart (n >= 5), a matrix's state is kept behind its packed form.
+TZG_HD int* schur_state(cfx* packed, int n) { return (int*)(packed + n * n - 1); }
 
 }  // namespace tzg

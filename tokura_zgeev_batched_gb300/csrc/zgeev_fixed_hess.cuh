@@ -258,10 +258,13 @@ __device__ __forceinline__ Reflector make_reflector(unsigned __int128 s, long lo
   return f;
 }
 
-template <int L, class Work, class Batch>
+// kQ: also forms the unitary Q of A = Q H Q^H (n x n column-major entries at q + where + slot * n^2; a row of Q is
+// one lane's, as a row of A from the right), leaves every matrix that is not reduced to the FP64 kernels, and keeps
+// the packed form n^2 entries apart, the state behind it (schur_state).
+template <int L, bool kQ, class Work, class Batch>
 __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, Batch B, cfx* __restrict__ hess,
                                                                      char* __restrict__ flag, int* __restrict__ state,
-                                                                     int one) {
+                                                                     cfx* __restrict__ q, int one) {
   constexpr int TW = L >= 32 ? 1 : 32 / L;
   extern __shared__ __align__(16) char fixed_smem[];
   const int slot = L >= 32 ? 0 : (threadIdx.x & 31) / L;
@@ -276,7 +279,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
   const Starts k = make_starts(one);
   int st = kStateDone;  // this matrix's state; only exponents go on to the reduction
   if (exists) {
-    if (!B.valid(j)) {
+    if (!kQ && !B.valid(j)) {
       const double nan = __longlong_as_double(0x7ff8000000000000LL);
       for (int i = G.rank; i < n; i += L) put_ev(B.out(j, n) + i, make_double2(nan, nan));
       if (G.rank == 0) flag[j] = (char)kInvalidInput;
@@ -291,7 +294,9 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
         A[c * ld + (e - c * n)] = cfx{__double_as_longlong(z.x), __double_as_longlong(z.y)};
       }
       emax = G.imax(emax);
-      if (emax == 0x7ff || emax == 0) {  // not finite, or zero
+      if (kQ && (emax == 0x7ff || emax == 0)) {
+        st = kStateGeneral;
+      } else if (emax == 0x7ff || emax == 0) {  // not finite, or zero
         const double v = emax != 0 ? __longlong_as_double(0x7ff8000000000000LL) : 0.0;
         for (int i = G.rank; i < n; i += L) put_ev(B.out(j, n) + i, make_double2(v, v));
         if (G.rank == 0) flag[j] = (char)(emax != 0 ? kNonFinite : kConverged);
@@ -335,10 +340,14 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
         st = lower == 0 || upper == 0 || spread > kFixedGradedBits ? kStateGeneral : emax - 1023 - p;
       }
     }
-    if (G.rank == 0) state[j] = st;
+    if (G.rank == 0) *(kQ ? schur_state(hess + tile.where + (long long)slot * nn, n) : state + j) = st;
   }
   const bool have = st != kStateDone && st != kStateGeneral;
   if (L > 32 ? !have : !__any_sync(0xffffffffu, have)) continue;  // block- or warp-uniform
+  cfx* const Q = kQ ? q + tile.where + (long long)slot * nn : nullptr;
+  if (kQ && have)
+    for (int c = 0; c < n; ++c)
+      for (int r = G.rank; r < n; r += L) Q[c * n + r] = cfx{r == c ? kFixedOne + kZero : kZero, kZero};
   G.sync();
 
   for (int r = 0; r + 1 < n; ++r) {
@@ -389,11 +398,12 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
     for (int q0 = 0; q0 < n; q0 += per2) {
       const int q = q0 + G.rank / qs;
       reflect_fixed<true>(k, A + (r + 1) * ld + q, ld, m, U, f.mur, f.mui, need && q < n, sub2, qs);
+      if (kQ) reflect_fixed<true>(k, Q + (r + 1) * n + q, n, m, U, f.mur, f.mui, need && q < n, sub2, qs);
     }
     G.sync();
   }
   if (have) {
-    cfx* const out = hess + tile.where + (long long)slot * hess_stride(n) + hess_lead(n);
+    cfx* const out = hess + tile.where + (long long)slot * (kQ ? nn : hess_stride(n)) + hess_lead(n);
     for (int c = 0; c < n; ++c)
       for (int r = G.rank; r <= min(c + 1, n - 1); r += L) out[hess_idx(r, c)] = A[c * ld + r];
   }

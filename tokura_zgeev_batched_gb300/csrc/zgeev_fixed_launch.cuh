@@ -15,17 +15,17 @@ inline cudaError_t allow_shared(Kernel kernel, size_t bytes) {
 
 // Staging and Hessenberg reduction of the matrices of `work`, of order n at most and `batch` of them at
 // most, in at most `max_blocks` blocks (0: no limit); a block takes several tiles then.
-template <int L, class Work, class Batch>
+template <int L, bool kQ = false, class Work, class Batch>
 inline cudaError_t launch_fixed_hess(const Work& work, int n, int batch, const Batch& B, cfx* hess, char* flag,
-                                     int* state, long long max_blocks, cudaStream_t stream) {
+                                     int* state, long long max_blocks, cudaStream_t stream, cfx* q = nullptr) {
   constexpr int tw = L >= 32 ? 1 : 32 / L;
   const size_t bytes = fixed_hess_shared<L>(n);
-  const cudaError_t err = allow_shared(fixed_hess_kernel<L, Work, Batch>, bytes);
+  const cudaError_t err = allow_shared(fixed_hess_kernel<L, kQ, Work, Batch>, bytes);
   if (err != cudaSuccess) return err;
   long long blocks = ((long long)batch + tw - 1) / tw;
   if (max_blocks > 0 && blocks > max_blocks) blocks = max_blocks;
-  fixed_hess_kernel<L, Work, Batch>
-      <<<(unsigned)blocks, L > 32 ? L : 32, bytes, stream>>>(work, B, hess, flag, state, 1);
+  fixed_hess_kernel<L, kQ, Work, Batch>
+      <<<(unsigned)blocks, L > 32 ? L : 32, bytes, stream>>>(work, B, hess, flag, state, q, 1);
   return cudaGetLastError();
 }
 

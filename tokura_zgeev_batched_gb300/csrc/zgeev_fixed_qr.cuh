@@ -171,18 +171,29 @@ struct FixedTile {
   int n, count;     // order, matrices (the slots 0 .. count - 1)
   long long j;      // this slot's matrix
   long long where;  // first entry of slot 0's packed form in the workspace (slots follow one another)
+  // Of the run of matrices of this order: its first entry where they are n^2 apart, its length, slot 0's position
+  // in it, and the matrices that a warp of the FP64 kernels takes together.
+  long long origin;
+  int total, pos, width;
 };
 
 // Work of a uniform batch: matrices 0 .. batch - 1 in order, `tw` to a tile.
+// `square`: n^2 entries apart in the workspace.
 struct UniformWork {
   int n, batch;
+  bool square = false;
+  int width = 32;
   __device__ __forceinline__ bool tile(long long t, int tw, int slot, FixedTile& out) const {
     const long long j0 = t * tw;
     if (j0 >= batch) return false;
     out.n = n;
     out.count = (int)min((long long)tw, batch - j0);
     out.j = j0 + slot;
-    out.where = j0 * hess_stride(n);
+    out.where = j0 * (square ? n * n : hess_stride(n));
+    out.origin = 0;
+    out.total = batch;
+    out.pos = (int)j0;
+    out.width = width;
     return true;
   }
 };

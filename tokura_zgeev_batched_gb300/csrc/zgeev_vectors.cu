@@ -8,6 +8,7 @@
 // of the triangular T, then VR = Q X and VL = Q Y, each column scaled like
 // LAPACK zgeev: unit 2-norm, component of largest modulus real and positive.
 #include "zgeev_backward.cuh"
+#include "zgeev_fixed_schur.cuh"
 #include "zgeev_internal.h"
 #include "zgeev_plain.cuh"
 
@@ -74,6 +75,18 @@ __device__ int vectors_prepare(const double2* __restrict__ src, double2* __restr
   return kPrepared;
 }
 
+// Eigenvectors from the Schur form.
+template <int L>
+__device__ __forceinline__ void vectors_of_schur(double2* __restrict__ VL, double2* __restrict__ VR, const BwdViews& V,
+                                                 const Group<L>& G) {
+  eigenvectors_of_t<L>(V, G);
+  if (VR) schur_vectors<L, true>(V, G, VR);
+  if (VL) schur_vectors<L, false>(V, G, VL);
+}
+
+// After the fixed-point Schur forms (zgeev_fixed_schur.cuh).
+constexpr int kPhaseFinish = 3;
+
 // Second half: Schur form with Q, eigenvalues, eigenvectors.
 template <int L>
 __device__ int vectors_finish(double2* __restrict__ w_out, double2* __restrict__ VL, double2* __restrict__ VR,
@@ -89,9 +102,7 @@ __device__ int vectors_finish(double2* __restrict__ w_out, double2* __restrict__
   }
   if (status != kConverged) return status;
   G.sync();
-  eigenvectors_of_t<L>(V, G);
-  if (VR) schur_vectors<L, true>(V, G, VR);
-  if (VL) schur_vectors<L, false>(V, G, VL);
+  vectors_of_schur<L>(VL, VR, V, G);
   return kConverged;
 }
 
@@ -112,6 +123,7 @@ __global__ void __launch_bounds__(128) zgeev_vectors_kernel(int n, int batch, co
   if (g0 >= batch) return;
   const int tw = (int)min((long long)TW, (long long)batch - g0);
   const int slot = lane / L;
+  const unsigned alive = __ballot_sync(0xffffffffu, slot < tw);
   if (slot >= tw) return;
   const Group<L> G;
   const long long nn = (long long)n * n;
@@ -124,7 +136,21 @@ __global__ void __launch_bounds__(128) zgeev_vectors_kernel(int n, int batch, co
   double2* vr = VR ? VR + j * nn : nullptr;
   const float2* e = est != nullptr ? est + j * n : nullptr;
   int status;
-  if (kPhase == kPhaseQR) {
+  if (kPhase == kPhaseFinish) {
+    const int st = take_schur<L>(G, alive, reinterpret_cast<cfx*>(work + region) + j * nn,
+                                 reinterpret_cast<const cfx*>(work + 2 * region) + j * nn, V.Q.p, n, tw);
+    if (st == kStateDone) return;  // not converged: eigenvalues and flag are written
+    if (st == kStateGeneral) {
+      int shift;
+      status = vectors_prepare<L>(A + j * nn, w + j * n, vl, vr, V, G, shift);
+      if (status == kPrepared)
+        status = vectors_finish<L>(w + j * n, vl, vr, V, G, itmax, shift, e, scaled_min_n);
+    } else {
+      G.sync();
+      vectors_of_schur<L>(vl, vr, V, G);
+      status = kConverged;
+    }
+  } else if (kPhase == kPhaseQR) {
     const int s = state[j];
     if (s == kStateDone) return;  // group-uniform
     status = vectors_finish<L>(w + j * n, vl, vr, V, G, itmax, s, e, scaled_min_n);
@@ -151,7 +177,7 @@ static cudaError_t launch_vectors_phase(int lanes, unsigned blocks, int threads,
                                         double2* work, char* flag, int itmax, const float2* est, int* state,
                                         int scaled_min_n) {
   const auto launch = [&](auto k) -> cudaError_t {
-    if (kPhase != kPhaseAll) {  // shared memory for the estimator running beside
+    if (kPhase != kPhaseAll && kPhase != kPhaseFinish) {  // shared memory for the estimator running beside
       const cudaError_t err =
           cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       if (err != cudaSuccess) return err;
@@ -174,12 +200,40 @@ static cudaError_t launch_vectors_phase(int lanes, unsigned blocks, int threads,
 // beside the first half (stage, Hessenberg, Q); without, first on `stream`.
 cudaError_t launch_vectors(int lanes, int n, int batch, const double2* A, double2* w, double2* VL, double2* VR,
                            double2* work, char* flag, int itmax, cudaStream_t stream, bool hints, const ForkJoin* fj,
-                           int scaled_min_n) {
+                           int scaled_min_n, bool fixed) {
   const int tw = 32 / lanes;
   const long long warps = ((long long)batch + tw - 1) / tw;
   const int threads = 32;  // one-warp blocks spread a resident batch evenly over the SMs
   const long long blocks = (warps * 32 + threads - 1) / threads;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+  if (fixed && n >= 5) {
+    // Schur forms in fixed point; with hints the estimator runs beside the Hessenberg reduction.
+    const size_t region = (size_t)n * n * batch;
+    const UniformWork list{n, batch, true, tw};
+    cfx* hess = reinterpret_cast<cfx*>(work + region);
+    cfx* q = reinterpret_cast<cfx*>(work + 2 * region);
+    const ContigBatch src{A, nullptr, n};
+    float2* est = nullptr;
+    cudaError_t err = cudaSuccess;
+    const bool beside = hints && fj != nullptr && fj->aux != nullptr;
+    std::unique_lock<std::mutex> lock;
+    if (beside) {
+      est = reinterpret_cast<float2*>(reinterpret_cast<char*>(work) + backward_workspace_bytes(n, batch));
+      lock = std::unique_lock<std::mutex>(*fj->mu);
+      if ((err = cudaEventRecord(fj->fork, stream)) != cudaSuccess) return err;
+      if ((err = cudaStreamWaitEvent(fj->aux, fj->fork, 0)) != cudaSuccess) return err;
+      if ((err = launch_estimates(n, batch, src, est, fj->aux)) != cudaSuccess) return err;
+      if ((err = cudaEventRecord(fj->join, fj->aux)) != cudaSuccess) return err;
+    }
+    if ((err = launch_schur_hess(list, n, batch, src, hess, q, 0, stream)) != cudaSuccess) return err;
+    if (beside && (err = cudaStreamWaitEvent(stream, fj->join, 0)) != cudaSuccess) return err;
+    const SchurDone done{work, nullptr, nullptr, nullptr, w, flag};
+    if ((err = launch_schur_qr(list, n, batch, EstimateShifts{est}, done, hess, q, itmax, 1, 0, stream)) !=
+        cudaSuccess)
+      return err;
+    return launch_vectors_phase<kPhaseFinish>(lanes, (unsigned)blocks, threads, stream, n, batch, A, w, VL, VR, work,
+                                              flag, itmax, nullptr, nullptr, scaled_min_n);
+  }
   if (!hints)
     return launch_vectors_phase<kPhaseAll>(lanes, (unsigned)blocks, threads, stream, n, batch, A, w, VL, VR, work,
                                            flag, itmax, nullptr, nullptr, scaled_min_n);
