@@ -96,8 +96,8 @@ TOKURA_API int tokuraGetPlainConfig(const tokurablas_t* handle, int n, int batch
 TOKURA_API int tokuraSetPlainQrLanes(tokurablas_t* handle, int n, int lanes_per_matrix);
 
 /* tokura_zgeev_batched_gpu on the FP64 kernels alone. The plain, layout,
- * host-buffer, workspace-free and ragged eigenvalue calls and the eigenvector
- * call start in 64-bit fixed point
+ * host-buffer, workspace-free and ragged eigenvalue calls, the eigenvector
+ * call and the ragged gradients start in 64-bit fixed point
  * (csrc/zgeev_fixed.cuh: the matrix as 64-bit integers with one exponent,
  * errors below the FP64 kernels' in norm; graded and triangular matrices are
  * left to those) unless the handle has a launch shape, rotation kind, shift

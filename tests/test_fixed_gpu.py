@@ -111,6 +111,60 @@ def test_ragged_gives_the_bits_of_the_uniform_calls(cuda, batch, lo_n, hi_n):
     assert err <= lo.TOL_REL_FRO * np.linalg.norm(mats[5])
 
 
+def ragged_backward(A, w, g, handle=None):
+    """A, w, g: tensors [batch, n, n], [batch, n], [batch, n]; through the ragged entry point."""
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    batch, n = w.shape
+    ns = torch.full((batch,), n, dtype=torch.int32, device="cuda")
+    offs = torch.arange(batch, dtype=torch.int64, device="cuda") * (n * n)
+    work = torch.empty(api.tokura_get_zgeev_ragged_backward_workspacesize(batch, A.numel()), dtype=torch.uint8,
+                       device="cuda")
+    A, w, g = A.contiguous(), w.contiguous(), g.contiguous()
+    gA, flag = torch.empty_like(A), torch.empty(batch, dtype=torch.int8, device="cuda")
+    h = handle if handle is not None else api.default_handle()
+    st = api.tokura_zgeev_ragged_backward_gpu(h, batch, ns.data_ptr(), offs.data_ptr(), None, A.numel(), A.data_ptr(),
+                                              w.data_ptr(), g.data_ptr(), gA.data_ptr(), work.data_ptr(),
+                                              flag.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    torch.cuda.synchronize()
+    return gA, flag
+
+
+@pytest.mark.parametrize("n", [4, 5, 8, 9, 16, 17, 24, 25, 32, 33, 48, 49, 64])
+def test_ragged_gradients_from_fixed_point_schur_forms(cuda, n):
+    """Against torch's gradient; matrices left to the FP64 kernel among the others."""
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A_np = wl.vdv(37, n, seed=5600 + n, min_sep=0.05)
+    A_np[3] = np.tril(A_np[3])  # triangular as stored
+    A_np[3] += np.diag(np.arange(n))  # well separated
+    Ac = torch.from_numpy(A_np).requires_grad_(True)
+    lam = torch.linalg.eigvals(Ac)
+    torch.sum(torch.exp(lam.real) + lam.real ** 2 + lam.imag ** 2).backward()
+    ref = Ac.grad.numpy()
+    A = torch.from_numpy(A_np).cuda()
+    w, f = api.zgeev_batched(A)
+    gbar = torch.exp(w.real) + 2 * w
+    g, fg = ragged_backward(A, w, gbar)
+    assert (fg == 0).all()
+    # relative error as the FP64 kernels are tested: 1e-9 on separated spectra
+    err = np.linalg.norm(g.cpu().numpy() - ref, axis=(1, 2)) / np.linalg.norm(ref, axis=(1, 2))
+    assert err.max() < 1e-9, err.max()
+    bad = A.clone()
+    bad[5, 1, 2] = complex("nan")
+    gb, fb = ragged_backward(bad, w, gbar)
+    assert fb[5] == 2 and torch.isnan(gb[5].real).all()
+    keep = [k for k in range(37) if k != 5]
+    assert torch.equal(torch.view_as_real(gb[keep]), torch.view_as_real(g[keep])) and (fb[keep] == 0).all()
+    lam_bad = w.clone()
+    lam_bad[6, 0] = complex("inf")  # first shifts that fixed point does not hold
+    gi, fi = ragged_backward(A, lam_bad, gbar)
+    assert torch.equal(torch.view_as_real(gi[7:]), torch.view_as_real(g[7:]))
+
+
 @pytest.mark.parametrize("n", [4, 5, 8, 9, 16, 17, 32, 33, 64])
 def test_eigenvectors_from_fixed_point_schur_forms(cuda, n):
     import torch
@@ -145,6 +199,9 @@ def test_schur_sweep_cap(cuda):
     assert h.set_sweep_cap(1) == 0
     w, VL, VR, f = api.zgeev_vectors(A, handle=h)
     assert (f == 1).all() and bool(torch.isfinite(torch.view_as_real(w)).all())
+    w0, _ = api.zgeev_batched(A)
+    g, fg = ragged_backward(A, torch.zeros_like(w0), w0, handle=h)  # useless first shifts
+    assert (fg == 1).all() and torch.isnan(g.real).all()
 
 
 def test_fp64_call_is_the_hinted_fp64_path(cuda):

@@ -248,7 +248,7 @@ extern "C" int tokura_zgeev_ragged_backward_gpu(tokurablas_t* handle, int batch_
       handle->ragged_lanes, handle->sm_count, batch_count, n, offsets, eig_offsets, total_elements,
       reinterpret_cast<const double2*>(A), reinterpret_cast<const double2*>(eigenvalues),
       reinterpret_cast<const double2*>(grad_eigenvalues), reinterpret_cast<double2*>(grad_A), work, flag,
-      handle->itmax_override, stream, handle->scaled_min_n);
+      handle->itmax_override, stream, handle->scaled_min_n, tzg::use_fixed_ragged_schur(handle), &handle->fj);
   return err == cudaSuccess ? 0 : 1;
 }
 

@@ -96,7 +96,7 @@ inline bool use_fixed(const tokurablas_t* h, int n) {
          h->scaled_min_n == kScaledRotationDefaultMinN && !h->shift_hints_set && h->balance_mode == 0;
 }
 
-// The same for the Schur forms of the eigenvectors (which no call balances).
+// The same for the Schur forms of gradients and eigenvectors (which no call balances).
 inline bool use_fixed_schur(const tokurablas_t* h, int n) {
   return h->plain[n].lanes == 0 && h->plain_qr_lanes[n] == 0 && h->scaled_min_n == kScaledRotationDefaultMinN &&
          !h->shift_hints_set;
@@ -106,6 +106,10 @@ inline bool use_fixed_schur(const tokurablas_t* h, int n) {
 inline bool use_fixed_ragged(const tokurablas_t* h) {
   return h->ragged_lanes == 0 && h->ragged_hint_min_n == kRaggedHintDefaultMinN &&
          h->scaled_min_n == kScaledRotationDefaultMinN && !h->shift_hints_set && h->balance_mode == 0;
+}
+
+inline bool use_fixed_ragged_schur(const tokurablas_t* h) {
+  return h->ragged_lanes == 0 && h->scaled_min_n == kScaledRotationDefaultMinN && !h->shift_hints_set;
 }
 
 inline PlainConfig plain_config_for(const tokurablas_t* h, int n, int batch) {

@@ -27,6 +27,7 @@
 //   5. Z = diag(gbar) X^H, M = Y Z in place, P = Q M, Abar = P Q^H (0.8 M).
 #pragma once
 
+#include "zgeev_fixed_qr.cuh"
 #include "zgeev_lane.cuh"
 #include "zgeev_scaled_qr.cuh"
 
@@ -37,7 +38,8 @@ namespace tzg {
 constexpr int kCloseEigenvalues = 4;
 
 // Relative deflation threshold of the gradient's Schur recomputation.
-constexpr double kGradDeflationTol = 100.0 * kUlp;
+constexpr int kGradDeflationUlps = 100;
+constexpr double kGradDeflationTol = kGradDeflationUlps * kUlp;
 
 struct BwdViews {
   MatView T, Q, XY;  // tile-interleaved n x n views (same layout as the forward's staging)
@@ -547,6 +549,25 @@ __device__ int backward_matrix(const double2* __restrict__ src, const double2* _
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
     for (int e = G.rank; e < n * n; e += L) gA[e] = make_double2(nan, nan);
     return status;
+  }
+  G.sync();
+  const bool close = eigenvectors_of_t<L>(V, G);
+  assemble_gradient<L>(V, G, gA);
+  return close ? kCloseEigenvalues : kConverged;
+}
+
+// The rest of a gradient whose Schur form is there (T's upper triangle, Q, the gradients in T's order in vec), from
+// the state of take_schur; kStateGeneral: all of it.
+template <int L>
+__device__ int backward_finish(int st, const double2* __restrict__ src, const double2* __restrict__ lam,
+                               const double2* __restrict__ gbar, double2* __restrict__ gA, const BwdViews& V,
+                               const Group<L>& G, int itmax, int scaled_min_n) {
+  if (st == kStateGeneral) return backward_matrix<L>(src, lam, gbar, gA, V, G, itmax, scaled_min_n);
+  const int n = V.T.n;
+  if (st == kStateDone) {  // not converged
+    const double nan = __longlong_as_double(0x7ff8000000000000LL);
+    for (int e = G.rank; e < n * n; e += L) gA[e] = make_double2(nan, nan);
+    return kNotConverged;
   }
   G.sync();
   const bool close = eigenvectors_of_t<L>(V, G);

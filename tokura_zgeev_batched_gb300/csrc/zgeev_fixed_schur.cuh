@@ -1,4 +1,4 @@
-// Schur forms A = Q T Q^H in 64-bit fixed point (zgeev_fixed.cuh), for the eigenvectors.
+// Schur forms A = Q T Q^H in 64-bit fixed point (zgeev_fixed.cuh), for ragged gradients and eigenvectors.
 //
 // The sweeps of zgeev_fixed_qr.cuh with every entry kept up to date: lane r of a matrix's L lanes holds the
 // indices j = r, r + L, ... of T. An index inside the window [lo, hi] is a column until its rotation is known

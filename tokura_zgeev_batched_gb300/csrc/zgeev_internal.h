@@ -59,7 +59,8 @@ size_t ragged_backward_workspace_bytes(int batch, long long total_elements);
 cudaError_t launch_ragged_backward(int lanes, int sms, int batch, const int* n, const long long* offsets,
                                    const long long* eig_offsets, long long total_elements, const double2* A,
                                    const double2* lam, const double2* gbar, double2* gA, void* work, char* flag,
-                                   int itmax_override, cudaStream_t stream, int scaled_min_n = 65);
+                                   int itmax_override, cudaStream_t stream, int scaled_min_n = 65, bool fixed = false,
+                                   const ForkJoin* fj = nullptr);
 
 // Eigenvalues with eigenvectors (workspace: backward_workspace_bytes).
 cudaError_t launch_vectors(int lanes, int n, int batch, const double2* A, double2* w, double2* VL, double2* VR,

@@ -6,7 +6,7 @@
 
 #include "zgeev_backward.cuh"
 #include "zgeev_estimate.cuh"
-#include "zgeev_fixed_qr.cuh"
+#include "zgeev_fixed_schur.cuh"
 #include "zgeev_internal.h"
 #include "zgeev_lane.cuh"
 #include "zgeev_scaled_qr.cuh"
@@ -90,7 +90,8 @@ struct RaggedArgs {
   const float2* est;     // forward: FP32 shift hints, kMaxN per matrix (or null)
   int* state;            // forward, split solve: pre-scaling exponent or kStateDone per matrix
   int est_min_n;         // forward: orders from which est holds hints
-  bool left_only = false;  // forward, after the fixed-point kernels: n = 1 and what they left (state)
+  // After the fixed-point kernels. Forward: only n = 1 and what they left (state); backward: from the Schur forms (n >= 5).
+  bool left_only = false;
   int scaled_min_n = 65;  // QR with scaled rotations from order max(7, lanes * scaled_min_n); > 64: never
 };
 
@@ -129,6 +130,7 @@ __device__ __forceinline__ void ragged_tile(const RaggedBin& bin, int t, const R
   const int slot = lane / L;
   const int u = t - bin.tile_start;
   const int tw = min(TW, bin.count - u * TW);
+  const unsigned alive = kBackward ? __ballot_sync(0xffffffffu, slot < tw) : 0u;
   if (slot >= tw) return;  // whole lane groups leave together
   const Group<L> G;
   const int nb = bin.n;
@@ -143,7 +145,13 @@ __device__ __forceinline__ void ragged_tile(const RaggedBin& bin, int t, const R
   if (kBackward) {
     BwdViews V{MatView{base, nb, tw}, MatView{base + a.region, nb, tw}, MatView{base + 2 * a.region, nb, tw},
                base + 3 * a.region, tw};
-    status = backward_matrix<L>(a.A + a.offsets[j], a.lam + a.eoff[j], a.gbar + a.eoff[j], a.gA + a.offsets[j], V,
+    int st = kStateGeneral;
+    if (a.left_only && nb >= 5) {  // warp-uniform
+      const long long mine = bin.stage + ((long long)u * TW + slot) * nn;
+      st = take_schur<L>(G, alive, reinterpret_cast<cfx*>(a.stage + a.region) + mine,
+                         reinterpret_cast<const cfx*>(a.stage + 2 * a.region) + mine, V.Q.p, nb, tw);
+    }
+    status = backward_finish<L>(st, a.A + a.offsets[j], a.lam + a.eoff[j], a.gbar + a.eoff[j], a.gA + a.offsets[j], V,
                                 G, itmax, scaled ? nb : kMaxN + 1);
   } else if (kPhase == kPhaseAll) {
     if (a.left_only && nb > 1 && a.state[j] != kStateGeneral) return;  // group-uniform

@@ -4,44 +4,9 @@
 //   second stream:                 \---- [orders 25..32 .. 2..4] --/
 // The classes above n = 32 keep their matrices in the workspace and the others in shared memory, so the two
 // streams' kernels fit on an SM together, and one's last, half-empty wave is filled by the other.
-#include "zgeev_fixed_launch.cuh"
-#include "zgeev_ragged.cuh"
+#include "zgeev_ragged_work.cuh"
 
 namespace tzg {
-
-// Matrices of orders nhi down to nlo; a tile holds matrices of one order.
-struct RaggedWork {
-  const RaggedPlan* plan;
-  const int* sorted;
-  int nhi, nlo;
-  __device__ __forceinline__ bool tile(long long t, int tw, int slot, FixedTile& out) const {
-    if (plan->overflow) return false;
-    for (int nb = nhi; nb >= nlo; --nb) {
-      const RaggedBin& bin = plan->bins[kMaxN - nb];
-      const int tiles = (bin.count + tw - 1) / tw;
-      if (t < tiles) {
-        const int p = (int)t * tw;
-        out.n = nb;
-        out.count = min(tw, bin.count - p);
-        out.j = slot < out.count ? sorted[bin.first + p + slot] : 0;
-        out.where = bin.stage + (long long)p * hess_stride(nb);
-        return true;
-      }
-      t -= tiles;
-    }
-    return false;
-  }
-};
-
-struct RaggedBatch {
-  const double2* A;
-  const long long* offsets;
-  const long long* eoff;
-  double2* eig;
-  __device__ __forceinline__ bool valid(long long) const { return true; }
-  __device__ __forceinline__ SrcContig src(long long j) const { return SrcContig{A + offsets[j]}; }
-  __device__ __forceinline__ double2* out(long long j, int) const { return eig + eoff[j]; }
-};
 
 cudaError_t ragged_launch_fixed(int sms, int batch, RaggedPlan* plan, const RaggedArgs& args, cudaStream_t stream,
                                 const ForkJoin* fj) {
