@@ -214,3 +214,58 @@ def test_fp64_call_is_the_hinted_fp64_path(cuda):
     assert h.set_shift_hints(1) == 0
     w1, f1 = api.zgeev_batched(A, handle=h)
     assert torch.equal(torch.view_as_real(w), torch.view_as_real(w1)) and (f == 0).all()
+
+
+def solve_real(A, handle=None):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    wr, wi, f = api.dgeev_batched(A, handle=handle)
+    torch.cuda.synchronize()
+    return torch.complex(wr, wi).cpu().numpy(), f.cpu().numpy()
+
+
+@pytest.mark.parametrize("n,batches", [(3, (9000, 60001)), (4, (12000, 40001)), (7, (4000, 30001)), (13, (2000, 9001)),
+                                       (21, (1100, 4000, 6001)), (30, (1100, 4001)), (33, (1001,)), (48, (1700, 8001)),
+                                       (61, (1001, 5001)), (64, (6001,))])
+def test_real_matrices_at_every_launch_shape(cuda, n, batches):
+    """The same bits in every shape; parity and conjugate pairs are checked on a slice."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(5700 + n)
+    A = torch.randn(max(batches), n, n, dtype=torch.float64, device="cuda", generator=gen)
+    few, f = solve_real(A[3:40])
+    rep = lo.real_parity_report(A[3:40].cpu().numpy(), few.real.copy(), few.imag.copy(), f)
+    assert rep["flag_mismatch"] == 0 and rep["pairs_ok"]
+    assert rep["max_rel_err_well"] <= lo.TOL_REL_FRO, rep["max_rel_err_well"]
+    for batch in batches:
+        w, f = solve_real(A[:batch])
+        assert (f == 0).all()
+        assert np.array_equal(w[3:40].view(np.uint64), few.view(np.uint64)), batch
+        tail = solve_real(A[batch - 6:batch])[0]
+        assert np.array_equal(w[-6:].view(np.uint64), tail.view(np.uint64)), batch
+
+
+@pytest.mark.parametrize("n", [3, 8, 20, 50])
+def test_real_matrices_left_to_fp64(cuda, n):
+    """Graded, triangular, and spectra whose conjugates can't be told apart."""
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A = np.random.default_rng(5800 + n).standard_normal((12, n, n))
+    d = 2.0 ** np.linspace(0, -40, n)
+    A[1] *= d[:, None] * d[None, :]
+    A[4] = np.triu(A[4])
+    A[7] = 1.0  # n - 1 zero eigenvalues
+    A[9] = A[9] @ np.diag(np.r_[2.0, 2.0, np.arange(n - 2)]) @ np.linalg.inv(A[9])  # a double one
+    A[10] = 0.0
+    A[11, 1, 2] = np.inf
+    At = torch.from_numpy(A).cuda()
+    w, f = solve_real(At)
+    h = api.Handle()
+    assert h.set_real_config(n, 8 if n >= 16 else 4, 32) == 0  # what so small a batch uses
+    w64, f64 = solve_real(At, h)
+    left = [1, 4, 7, 9]
+    assert np.array_equal(w[left].view(np.uint64), w64[left].view(np.uint64))
+    assert np.array_equal(f, f64) and f[11] == 2
+    assert (w[10] == 0).all() and np.isnan(w[11].real).all()

@@ -112,6 +112,11 @@ inline bool use_fixed_ragged_schur(const tokurablas_t* h) {
   return h->ragged_lanes == 0 && h->scaled_min_n == kScaledRotationDefaultMinN && !h->shift_hints_set;
 }
 
+// The same for real matrices (a launch shape or balancing on the handle names the FP64 kernel).
+inline bool use_fixed_real(const tokurablas_t* h, int n) {
+  return n > 2 && h->real[n].lanes == 0 && h->real[n].threads == 0 && h->balance_mode == 0;
+}
+
 inline PlainConfig plain_config_for(const tokurablas_t* h, int n, int batch) {
   PlainConfig c = h->plain[n];
   if (use_fixed(h, n)) c.fixed = h->sm_count;

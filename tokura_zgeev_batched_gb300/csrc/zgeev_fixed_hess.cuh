@@ -225,7 +225,8 @@ struct Reflector {
 
 TZG_HD long long shift_by(long long v, int q) { return q >= 0 ? v << q : v >> -q; }
 
-__device__ __forceinline__ Reflector make_reflector(unsigned __int128 s, long long x0r, long long x0i) {
+// The part that a real column needs too (its imaginary part does not enter here).
+__device__ __forceinline__ Reflector make_real_reflector(unsigned __int128 s, long long x0r) {
   Reflector f;
   const unsigned long long shi = (unsigned long long)(s >> 64), slo = (unsigned long long)s;
   const int p = shi ? 127 - clz64(shi) : 63 - clz64(slo);
@@ -238,8 +239,8 @@ __device__ __forceinline__ Reflector make_reflector(unsigned __int128 s, long lo
     mid = mad_wide(t.l, g.h, mid);
     f.nn = (mad_wide(t.h, g.h, 0) << 4) + (mid >> 28);
   }
-  const long long xr = shift_by(x0r, f.q), xi = shift_by(x0i, f.q);
-  const long long a = f.nn + (xr < 0 ? -xr : xr), b = xr < 0 ? -xi : xi;
+  const long long xr = shift_by(x0r, f.q);
+  const long long a = f.nn + (xr < 0 ? -xr : xr);
   const long long beta = f.q >= 1 ? ((f.nn >> (f.q - 1)) + 1) >> 1 : f.nn << -f.q;
   f.beta = xr < 0 ? beta : -beta;
   {  // ||x - beta e1||^2 = 2 N (N + |Re x0|)
@@ -251,6 +252,13 @@ __device__ __forceinline__ Reflector make_reflector(unsigned __int128 s, long lo
     const long long g4 = inv_sqrt(low ? (hh << 4) + (mid >> 28) : (hh << 2) + (mid >> 30));
     f.gv = limbs(low ? g4 << 1 : g4);
   }
+  return f;
+}
+
+__device__ __forceinline__ Reflector make_reflector(unsigned __int128 s, long long x0r, long long x0i) {
+  Reflector f = make_real_reflector(s, x0r);
+  const long long xr = shift_by(x0r, f.q), xi = shift_by(x0i, f.q);
+  const long long a = f.nn + (xr < 0 ? -xr : xr), b = xr < 0 ? -xi : xi;
   const RotC c = make_rotc(a >> 1, 0, b >> 1);  // mu = 2 cos(phi) exp(-i phi), tan(phi) = b / a
   const long long cc = value(c.cr), ss = value(c.s);
   f.mur = limbs((long long)(((__int128)cc * cc) >> 62) | 1);

@@ -54,22 +54,12 @@ inline cudaError_t launch_fixed_qr(const Work& work, int n, int batch, const Bat
 // Above n = 32 shared memory holds few matrices (6 per SM at n = 64), so batches of more than those
 // stay in the workspace, which the caches hold: n = 64, 8,192 matrices 57.7 ms in shared memory, 46 ms so
 // (304 matrices: 4.9 against 6.1 ms); n = 48, 20,000 matrices 52.5 ms at 16 lanes, 56.6 at 32.
+// Real matrices leave scratch for the complex iterates of 4 in 9 of them, used from 1.7 times the matrices that shared
+// memory holds: n = 64, 3,000 matrices 18.7 ms so (1,300 blocks) and 17.1 in shared memory (912), 6,000 25.8 and 30.8,
+// 16,384 62.0 and 81.9; n = 47, 20,000 39.2 and 40.8; n = 40, 5,000 9.0 and 7.4.
 template <class Batch>
-cudaError_t launch_fixed(int n, int batch, int sms, const Batch& B, cfx* hess, char* flag, int itmax, int* state,
-                         cudaStream_t stream) {
-  cudaError_t err;
-  const UniformWork work{n, batch};
-  if (n <= 4)
-    err = launch_fixed_hess<4>(work, n, batch, B, hess, flag, state, 0, stream);
-  else if (n <= 8)
-    err = launch_fixed_hess<8>(work, n, batch, B, hess, flag, state, 0, stream);
-  else if (n <= 16)
-    err = launch_fixed_hess<16>(work, n, batch, B, hess, flag, state, 0, stream);
-  else if (n <= 32)
-    err = launch_fixed_hess<32>(work, n, batch, B, hess, flag, state, 0, stream);
-  else
-    err = launch_fixed_hess<128>(work, n, batch, B, hess, flag, state, 0, stream);
-  if (err != cudaSuccess) return err;
+cudaError_t launch_fixed_shape(const UniformWork& work, int n, int batch, int sms, const Batch& B, cfx* hess,
+                               char* flag, int itmax, int* state, cudaStream_t stream) {
   // Whether a batch is small enough for `lanes` lanes per matrix and `warps` warps per SM.
   auto fits = [&](int lanes, int warps) { return (long long)batch * lanes <= (long long)sms * 32 * warps; };
 #define TZG_FIXED_QR(L, T, G, BLOCKS) \
@@ -96,10 +86,35 @@ cudaError_t launch_fixed(int n, int batch, int sms, const Batch& B, cfx* hess, c
   }
   // Matrices that shared memory holds on all SMs (228 KB each, 1 KB of it reserved per block).
   const long long resident = (long long)sms * (233472 / (fixed_qr_shared<32, false>(n) + 1024));
-  if (batch <= resident) TZG_FIXED_QR(32, 2, false, 0);
-  if (n <= 48 && !fits(16, 12)) TZG_FIXED_QR(16, 4, true, sms * 12);
-  TZG_FIXED_QR(32, 2, true, sms * 24);
+  if constexpr (kRealBatch<Batch>) {
+    const long long blocks = min((long long)sms * 24, (B.room - qr_slack(n)) / (hess_count(n) + 2));
+    if (10 * blocks < 17 * resident) TZG_FIXED_QR(32, 2, false, 0);
+    TZG_FIXED_QR(32, 2, true, blocks);
+  } else {
+    if (batch <= resident) TZG_FIXED_QR(32, 2, false, 0);
+    if (n <= 48 && !fits(16, 12)) TZG_FIXED_QR(16, 4, true, sms * 12);
+    TZG_FIXED_QR(32, 2, true, sms * 24);
+  }
 #undef TZG_FIXED_QR
+}
+
+template <class Batch>
+cudaError_t launch_fixed(int n, int batch, int sms, const Batch& B, cfx* hess, char* flag, int itmax, int* state,
+                         cudaStream_t stream) {
+  cudaError_t err;
+  const UniformWork work{n, batch};
+  if (n <= 4)
+    err = launch_fixed_hess<4>(work, n, batch, B, hess, flag, state, 0, stream);
+  else if (n <= 8)
+    err = launch_fixed_hess<8>(work, n, batch, B, hess, flag, state, 0, stream);
+  else if (n <= 16)
+    err = launch_fixed_hess<16>(work, n, batch, B, hess, flag, state, 0, stream);
+  else if (n <= 32)
+    err = launch_fixed_hess<32>(work, n, batch, B, hess, flag, state, 0, stream);
+  else
+    err = launch_fixed_hess<128>(work, n, batch, B, hess, flag, state, 0, stream);
+  if (err != cudaSuccess) return err;
+  return launch_fixed_shape(work, n, batch, sms, B, hess, flag, itmax, state, stream);
 }
 
 }  // namespace tzg

@@ -67,6 +67,45 @@ __device__ __forceinline__ double fixed_to_double(long long w, int e) {
   return __longlong_as_double((long long)(sign | (((unsigned long long)(ex - 1) << 52) + r)));
 }
 
+// Batches of real matrices (n >= 3). Their workspace, n^2 words of 8 bytes for each, holds for each its packed real
+// Hessenberg form and a word with its state, one after another, and behind these `scratch`: room for the complex
+// iterates of some of them at a time. Eigenvalues go to wr and wi; flag is kLeftToFp64 for a matrix that the
+// FP64 kernel solves.
+constexpr char kLeftToFp64 = 100;
+struct RealBatch {
+  const long long* packed;
+  void* wr;
+  void* wi;
+  bool single;
+  cfx* scratch;
+  long long room;  // of scratch, in entries
+  __device__ __forceinline__ void put(long long i, double re, double im) const {
+    if (single) {
+      static_cast<float*>(wr)[i] = (float)re;
+      static_cast<float*>(wi)[i] = (float)im;
+    } else {
+      static_cast<double*>(wr)[i] = re;
+      static_cast<double*>(wi)[i] = im;
+    }
+  }
+};
+template <class Batch>
+constexpr bool kRealBatch = false;
+template <>
+constexpr bool kRealBatch<RealBatch> = true;
+__host__ __device__ constexpr int real_words(int n) { return hess_count(n) + 1; }
+// Eigenvalues of a real matrix are conjugates of each other, or real, if they are so to this many units (2^-30 of the
+// norm). Where that leaves a choice (two of them closer than this), or finds no partner, the FP64 kernel, whose
+// iteration keeps conjugates, solves the matrix.
+constexpr long long kConjugateUnits = 1LL << 31;
+__device__ __forceinline__ bool conjugates(cfx a, cfx b) {
+  return mag64(a.x - b.x) <= (unsigned long long)kConjugateUnits &&
+         mag64(a.y - kZero + (b.y - kZero)) <= (unsigned long long)kConjugateUnits;
+}
+__device__ __forceinline__ bool nearly_real(cfx a) {
+  return mag64(a.y - kZero) <= (unsigned long long)(kConjugateUnits / 2);
+}
+
 // Everything a lane keeps during a sweep. What bounds it: the 32x32-bit multiplier, one warp
 // instruction in four clocks of a sub-partition (a rotation is 36 of them, its coefficients 22), 60 % busy
 // at n = 16 (65,536 matrices, 9 warps per SM) and 50 % at n = 64 in shared memory (5.4 warps per SM); the rest is
@@ -214,12 +253,31 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
   const int itmax = itmax0 > 0 ? itmax0 : default_itmax(n);
   const long long j = tile.j;
   // Whole warps stay together; lanes without a matrix keep an empty window.
-  const int st = slot < tile.count ? state[j] : kStateDone;
+  constexpr bool kReal = kRealBatch<Batch>;
+  int st = kStateDone;
+  if (slot < tile.count) {
+    if constexpr (kReal)
+      st = (int)B.packed[(j + 1) * real_words(n) - 1];
+    else
+      st = state[j];
+  }
   const bool have = st != kStateDone && st != kStateGeneral;
   if (!__any_sync(kAll, have)) continue;
   cfx* H;
   cfx* words = reinterpret_cast<cfx*>(fixed_smem);
-  if (kGlobal) {
+  if constexpr (kReal) {
+    if (kGlobal) {
+      H = B.scratch + ((long long)blockIdx.x * TW + slot) * (count + 2) + 1;
+    } else {
+      H = words + 1 + slot * stride;
+      words += TW * stride;
+    }
+    if (have) {
+      const long long* const src = B.packed + j * real_words(n);
+      for (int e = rank; e < count; e += L) H[e] = cfx{src[e], kZero};
+    }
+    __syncwarp();
+  } else if (kGlobal) {
     H = hess + tile.where + (long long)min(slot, tile.count - 1) * hess_stride(n) + 1;
   } else {
     cfx* const sm = words + 1;
@@ -244,6 +302,7 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
 
   int hi = have ? n - 1 : -1;
   int its = 0, kdefl = 0, status = kConverged;
+  bool follow = false;  // a real matrix's next shift is the conjugate of the eigenvalue below the window
 #ifdef TOKURA_DEBUG_BOUNDS
   int sweeps = 0;
 #endif
@@ -277,6 +336,10 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
       const unsigned long long below = small & ((2ull << hi) - 1ull);
       lo = below ? 63 - clz64(below) : 0;
       if (lo < hi) break;
+      if (kReal) {
+        const cfx d = H[hess_idx(hi, hi)];
+        follow = !nearly_real(d) && !(follow && conjugates(d, H[hess_idx(hi + 1, hi + 1)]));
+      }
       // Converged: row hi becomes the (zero) row under the next window.
       if (rank == 0) H[hess_idx(hi, hi - 1)] = cfx{kZero, kZero};
       --hi;
@@ -306,6 +369,10 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
         sigma.x = f.x - kZero;
         sigma.x += sigma.x < 0 ? h : -h;
         sigma.y = f.y - kZero;
+      } else if (kReal && follow && its == 1) {
+        const cfx e = H[hess_idx(hi + 1, hi + 1)];
+        sigma.x = e.x - kZero;
+        sigma.y = kZero - e.y;
       } else {
         const cfx b = H[hess_idx(hi - 1, hi)];
         const cfx e = wilkinson_correction(H[hess_idx(hi - 1, hi - 1)], cfx{b.x - kZero, b.y - kZero},
@@ -356,7 +423,57 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
     if (m > 0 && rank == 0) H[hess_idx(lo, lo - 1)] = cfx{kZero, kZero};
     __syncwarp();
   }
-  if (have) {
+  if constexpr (kReal) {
+    // Pairs, in the order of their first members. Anything unclear is left to the FP64 kernel.
+    unsigned long long reals = 0, leads = 0;
+    bool clear = status == kConverged;
+    int partner[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const int i = rank + t * L;
+      int found = 0;
+      partner[t] = i;
+      if (have && i < n) {
+        const cfx d = H[hess_idx(i, i)];
+        for (int c = 0; c < n; ++c)
+          if (c != i && conjugates(d, H[hess_idx(c, c)])) {
+            ++found;
+            partner[t] = c;
+          }
+        clear = clear && found == (nearly_real(d) ? 0 : 1);
+      }
+      const bool one = have && i < n && found == 0, lead = have && i < n && partner[t] > i;
+      if (L == 1) {
+        reals |= (unsigned long long)one << i;
+        leads |= (unsigned long long)lead << i;
+      } else {
+        const unsigned part = L == 32 ? kAll : (1u << (L & 31)) - 1u;
+        reals |= (unsigned long long)((__ballot_sync(kAll, one) >> base) & part) << (t * L);
+        leads |= (unsigned long long)((__ballot_sync(kAll, lead) >> base) & part) << (t * L);
+      }
+    }
+    const unsigned unclear = __ballot_sync(kAll, !clear) >> base;
+    clear = (L == 32 ? unclear : unclear & ((1u << (L & 31)) - 1u)) == 0;
+    if (have && clear) {
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const int i = rank + t * L, p = partner[t];
+        if (i >= n || p < i) continue;
+        const unsigned long long before = (1ull << i) - 1ull;
+        const long long at = j * n + __popcll(reals & before) + 2 * __popcll(leads & before);
+        const cfx d = H[hess_idx(i, i)], e = H[hess_idx(p, p)];
+        if (p == i) {
+          B.put(at, fixed_to_double(d.x - kZero, st), 0.0);
+        } else {
+          const double re = fixed_to_double(d.x - kZero + (e.x - kZero), st - 1);
+          const double im = fabs(fixed_to_double(d.y - e.y, st - 1));
+          B.put(at, re, im);
+          B.put(at + 1, re, -im);
+        }
+      }
+    }
+    if (have && rank == 0) flag[j] = clear ? (char)kConverged : kLeftToFp64;
+  } else if (have) {
     for (int i = rank; i < n; i += L) {
       const cfx d = H[hess_idx(i, i)];
       put_ev(B.out(j, n) + i, make_double2(fixed_to_double(d.x - kZero, st), fixed_to_double(d.y - kZero, st)));
