@@ -122,9 +122,11 @@ TZG_HD float addf(float a, float b) {
   return a + b;
 #endif
 }
-TZG_HD float rsqrt_seed(float x) {
+TZG_HD float rsqrt_seed(float x) {  // x normal
 #ifdef __CUDA_ARCH__
-  return rsqrtf(x);
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 #else
   return 1.0f / sqrtf(x);
 #endif
@@ -198,8 +200,13 @@ struct RotC {
   Limbs cr, ci, s;
 };
 TZG_HD RotC make_rotc(long long xr, long long xi, long long y) {
-  xr += (xr | xi | y) == 0 ? 1 : 0;
-  const int z = clz64(mag64(xr) | mag64(xi) | mag64(y) | 1ull) - 2;
+  // Only for values below 2^-30 of the bound do the low words and zeros matter.
+  const unsigned top = mag32(high(xr)) | mag32(high(xi)) | mag32(high(y));
+  int z = clz32(top) - 2;
+  if (top == 0) {
+    xr += (xr | xi | y) == 0 ? 1 : 0;
+    z = clz64(mag64(xr) | mag64(xi) | mag64(y) | 1ull) - 2;
+  }
   const Limbs a = limbs(xr << z), b = limbs(xi << z), d = limbs(y << z);  // the largest's top bit at 2^61
   long long mid = mad_wide(a.h, a.l, 0);
   long long T = mad_wide(a.h, a.h, 0);

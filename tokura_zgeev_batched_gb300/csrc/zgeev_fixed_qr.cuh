@@ -93,7 +93,7 @@ template <class Batch>
 constexpr bool kRealBatch = false;
 template <>
 constexpr bool kRealBatch<RealBatch> = true;
-__host__ __device__ constexpr int real_words(int n) { return hess_count(n) + 1; }
+TZG_HD int real_words(int n) { return hess_count(n) + 1; }
 // Eigenvalues of a real matrix are conjugates of each other, or real, if they are so to this many units (2^-30 of the
 // norm). Where that leaves a choice (two of them closer than this), or finds no partner, the FP64 kernel, whose
 // iteration keeps conjugates, solves the matrix.
