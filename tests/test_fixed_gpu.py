@@ -226,7 +226,7 @@ def solve_real(A, handle=None):
 
 
 @pytest.mark.parametrize("n,batches", [(3, (9000, 60001)), (4, (12000, 40001)), (7, (4000, 30001)), (13, (2000, 9001)),
-                                       (21, (1100, 4000, 6001)), (30, (1100, 4001)), (33, (1001,)), (48, (1700, 8001)),
+                                       (21, (1100, 4000, 6001)), (30, (1100, 4001)), (33, (1001,)), (40, (12001,)), (48, (1700, 8001)),
                                        (61, (1001, 5001)), (64, (6001,))])
 def test_real_matrices_at_every_launch_shape(cuda, n, batches):
     """The same bits in every shape; parity and conjugate pairs are checked on a slice."""

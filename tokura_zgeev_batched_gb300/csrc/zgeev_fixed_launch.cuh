@@ -53,10 +53,14 @@ inline cudaError_t launch_fixed_qr(const Work& work, int n, int batch, const Bat
 //   n = 32: 10,000 matrices 9.0 / 8.0 / 9.8 at 8 / 16 / 32, 1,000 2.1 / 1.6 / 1.5.
 // Above n = 32 shared memory holds few matrices (6 per SM at n = 64), so batches of more than those
 // stay in the workspace, which the caches hold: n = 64, 8,192 matrices 57.7 ms in shared memory, 46 ms so
-// (304 matrices: 4.9 against 6.1 ms); n = 48, 20,000 matrices 52.5 ms at 16 lanes, 56.6 at 32.
+// (304 matrices: 4.9 against 6.1 ms). 32 lanes run best in 24 warps per SM (16,384 of n = 64: 92.0 / 88.0 / 87.2 / 97.9 ms
+// at 16 / 20 / 24 / 32), 16 lanes in as many as 128 registers or, from about 85 MB, the L2 cache allow: 12 / 14 / 16 warps
+// 39.0 / 38.5 / 35.6 (30,000 of n = 36), 37.8 / 36.8 / 36.4 (20,000 of 42), 53.3 / 52.2 / 52.8 (20,000 of 48; 32 lanes 55.7),
+// 94.4 / 93.0 / 95.5 (16,384 of 64).
 // Real matrices leave scratch for the complex iterates of 4 in 9 of them, used from 1.7 times the matrices that shared
 // memory holds: n = 64, 3,000 matrices 18.7 ms so (1,300 blocks) and 17.1 in shared memory (912), 6,000 25.8 and 30.8,
-// 16,384 62.0 and 81.9; n = 47, 20,000 39.2 and 40.8; n = 40, 5,000 9.0 and 7.4.
+// 16,384 62.0 and 81.9. At 16 lanes they need 32 matrices per SM to gain: n = 42, 9,000 matrices 14.0 and 13.8, 15,000 20.5
+// and 22.9, 30,000 37.8 and 45.3; n = 48, 15,000 28.5 and 30.2.
 template <class Batch>
 cudaError_t launch_fixed_shape(const UniformWork& work, int n, int batch, int sms, const Batch& B, cfx* hess,
                                char* flag, int itmax, int* state, cudaStream_t stream) {
@@ -86,13 +90,16 @@ cudaError_t launch_fixed_shape(const UniformWork& work, int n, int batch, int sm
   }
   // Matrices that shared memory holds on all SMs (228 KB each, 1 KB of it reserved per block).
   const long long resident = (long long)sms * (233472 / (fixed_qr_shared<32, false>(n) + 1024));
+  const int warps16 = n <= 42 ? 16 : 14;  // per SM, at 16 lanes
   if constexpr (kRealBatch<Batch>) {
-    const long long blocks = min((long long)sms * 24, (B.room - qr_slack(n)) / (hess_count(n) + 2));
+    const long long places = (B.room - qr_slack(n)) / (hess_count(n) + 2);
+    if (n <= 48 && places >= sms * 32LL) TZG_FIXED_QR(16, 4, true, sms * warps16);
+    const long long blocks = min((long long)sms * 24, places);
     if (10 * blocks < 17 * resident) TZG_FIXED_QR(32, 2, false, 0);
     TZG_FIXED_QR(32, 2, true, blocks);
   } else {
     if (batch <= resident) TZG_FIXED_QR(32, 2, false, 0);
-    if (n <= 48 && !fits(16, 12)) TZG_FIXED_QR(16, 4, true, sms * 12);
+    if (n <= 48 && !fits(16, 12)) TZG_FIXED_QR(16, 4, true, sms * warps16);
     TZG_FIXED_QR(32, 2, true, sms * 24);
   }
 #undef TZG_FIXED_QR
