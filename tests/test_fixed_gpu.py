@@ -84,7 +84,7 @@ def test_extreme_scales_and_exact_rows(cuda):
         assert np.array_equal(np.ldexp(ws.view(np.float64), -e), w.view(np.float64))
 
 
-@pytest.mark.parametrize("batch,lo_n,hi_n", [(40, 1, 64), (700, 1, 64), (2500, 1, 33), (6000, 1, 17)])
+@pytest.mark.parametrize("batch,lo_n,hi_n", [(40, 1, 64), (700, 1, 64), (2500, 1, 33), (6000, 1, 17), (31000, 32, 34)])
 def test_ragged_gives_the_bits_of_the_uniform_calls(cuda, batch, lo_n, hi_n):
     """Few and many matrices (both sets of launch shapes), every order, a graded one among them."""
     import torch

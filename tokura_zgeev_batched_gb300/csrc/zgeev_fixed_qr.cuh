@@ -109,8 +109,9 @@ __device__ __forceinline__ bool nearly_real(cfx a) {
 // Everything a lane keeps during a sweep. What bounds it: the 32x32-bit multiplier, one warp
 // instruction in four clocks of a sub-partition (a rotation is 36 of them, its coefficients 22), 60 % busy
 // at n = 16 (65,536 matrices, 9 warps per SM) and 50 % at n = 64 in shared memory (5.4 warps per SM); the rest is
-// the chain of a step with few warps to hide it. Making rotation k + 1 beside step k's work (18 more
-// multiplications) was 8 % faster at n >= 32 with the matrices in shared memory, 15-25 % slower below.
+// the chain of a step with few warps to hide it. Making rotation k + 1 beside step
+// k's work (18 more multiplications and two more loads in every lane) was slower: 16,384 matrices of n = 64 87.2 -> 116.5
+// ms, 10,000 of n = 32 7.9 -> 9.0.
 template <int L, int T>
 struct QrLane {
   cfx* H;          // packed matrix

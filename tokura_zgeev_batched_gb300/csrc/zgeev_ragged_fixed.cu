@@ -34,7 +34,13 @@ cudaError_t ragged_launch_fixed(int sms, int batch, RaggedPlan* plan, const Ragg
   TZG_HESS(64, 49, 128, stream);
   TZG_HESS(48, 33, 128, stream);
   TZG_QR(64, 49, 32, 2, true, (long long)sms * 24, stream);
-  TZG_QR(48, 33, 32, 2, true, (long long)sms * 24, stream);
+  // Orders 33 to 48 at 32 and 16 lanes: 20,000 orders in U{1..64} 45.5 and 47.1 ms, 30,000 63.3 and 63.3, 40,000 81.6 and
+  // 79.2, 200,000 396 and 368 (more lanes while the class is a wave or two).
+  if (batch < sms * 200) {
+    TZG_QR(48, 33, 32, 2, true, (long long)sms * 24, stream);
+  } else {
+    TZG_QR(48, 33, 16, 4, true, (long long)sms * 14, stream);
+  }
   TZG_HESS(32, 25, 32, side);
   TZG_HESS(24, 17, 32, side);
   TZG_HESS(16, 9, 16, side);
