@@ -269,3 +269,13 @@ def test_real_matrices_left_to_fp64(cuda, n):
     assert np.array_equal(w[left].view(np.uint64), w64[left].view(np.uint64))
     assert np.array_equal(f, f64) and f[11] == 2
     assert (w[10] == 0).all() and np.isnan(w[11].real).all()
+
+
+@pytest.mark.parametrize("n,batch", [(5, 8191), (5, 29183), (12, 30001)])
+def test_host_chunks_solved_in_turn_give_the_device_call(cuda, n, batch):
+    from tokura_zgeev_batched_gb300 import api
+
+    A = wl.torch_gaussian(batch, n, seed=5900 + batch)
+    w, f = api.zgeev_batched_host(A.cpu())
+    wd, fd = solve(A)
+    assert np.array_equal(np.ascontiguousarray(w).view(np.uint64), wd.view(np.uint64)) and np.array_equal(f, fd)

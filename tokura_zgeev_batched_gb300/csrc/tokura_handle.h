@@ -16,6 +16,7 @@ struct HostPipeline {
   char* d_flag[kStreams] = {};
   cudaStream_t stream[kStreams] = {};
   cudaEvent_t copied[kStreams] = {};  // end of the host-to-device copy last issued on each stream
+  cudaEvent_t solved[kStreams] = {};  // end of a chunk's solve (chunks solved one after another)
   cudaEvent_t copy_begin = nullptr, copy_end = nullptr;  // timing of one call's host-to-device copies
   double link_gbs = 0.0;  // host-to-device rate seen by the last call (GB/s; 0 = not measured yet)
   double link_gbs_fixed = 0.0;  // rate set by tokuraSetHostLinkRate (> 0 replaces the measured one)
