@@ -3,7 +3,10 @@
 //   caller's stream: [planning] --fork-- [orders 49..64, 33..48] --join-- [FP64: what was left]
 //   second stream:                 \---- [orders 25..32 .. 2..4] --/
 // The classes above n = 32 keep their matrices in the workspace and the others in shared memory, so the two
-// streams' kernels fit on an SM together, and one's last, half-empty wave is filled by the other.
+// streams' kernels fit on an SM together, and one's last, half-empty wave is filled by the other. From 100 matrices per
+// SM on the waves are many and what the two evict from each other's caches costs more: all on the caller's
+// stream. Orders in U{1..64}, two streams and one: 1,000 matrices 9.6 and 12.0 ms, 4,000 13.0 and 14.2, 9,000 22.7 and 20.3,
+// 13,000 24.0 and 26.2, 20,000 45.4 and 37.2, 60,000 117 and 100, 200,000 397 and 319.
 #include "zgeev_ragged_work.cuh"
 
 namespace tzg {
@@ -13,7 +16,7 @@ cudaError_t ragged_launch_fixed(int sms, int batch, RaggedPlan* plan, const Ragg
   const RaggedBatch B{args.A, args.offsets, args.eoff, args.eig};
   cfx* hess = reinterpret_cast<cfx*>(args.stage);
   const int itmax = args.itmax_override;
-  const bool two = fj != nullptr && fj->aux != nullptr;
+  const bool two = batch < sms * 100 && fj != nullptr && fj->aux != nullptr;
   cudaError_t err = cudaSuccess;
   cudaStream_t side = stream;
   if (two) {
@@ -34,8 +37,8 @@ cudaError_t ragged_launch_fixed(int sms, int batch, RaggedPlan* plan, const Ragg
   TZG_HESS(64, 49, 128, stream);
   TZG_HESS(48, 33, 128, stream);
   TZG_QR(64, 49, 32, 2, true, (long long)sms * 24, stream);
-  // Orders 33 to 48 at 32 and 16 lanes: 20,000 orders in U{1..64} 45.5 and 47.1 ms, 30,000 63.3 and 63.3, 40,000 81.6 and
-  // 79.2, 200,000 396 and 368 (more lanes while the class is a wave or two).
+  // Orders 33 to 48 at 32 and 16 lanes: 20,000 orders in U{1..64} 37.2 and 38.6 ms, 30,000 53.4 and 52.7, 60,000 102.3 and
+  // 99.5, 200,000 331 and 319 (more lanes while the class is a wave or two).
   if (batch < sms * 200) {
     TZG_QR(48, 33, 32, 2, true, (long long)sms * 24, stream);
   } else {
