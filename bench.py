@@ -36,9 +36,16 @@ SEED = 20261203
 SWEEP_NS = (4, 8, 16, 32, 48)  # the size sweep's other orders (n = 64 is the timed workload)
 
 
-# Orders from which the plain entry point runs with FP32 shift hints by default
-# (three kernels per call: estimator, Hessenberg phase, QR phase).
+# A plain call with the library's choices is three kernels: Hessenberg reduction and QR in 64-bit
+# fixed point, and the FP64 kernel for the matrices that these leave. With a launch shape set
+# (--lanes) it is the FP64 path: an FP32 estimator, the Hessenberg phase and the QR phase from n = 12 on.
 SHIFT_HINT_MIN_N = 12
+
+
+def launches_per_call(n: int, lanes: int) -> int:
+    if lanes:
+        return 3 if n >= SHIFT_HINT_MIN_N else 1
+    return 3 if n > 1 else 1
 
 
 def set_workload(n: int, batch: int = 0) -> None:
@@ -815,8 +822,8 @@ def measure_ragged(h, dev, stream, peak, batch: int = 200000) -> dict:
                                    f"matrix ({ms_conc_capped:.1f} ms, flags equal: {capped_flags_same})",
             "fp64_frac": work_flops / (best * 1e-3) / peak, "flagged": flagged,
             "plain_launches": int(np.count_nonzero(counts)), "parity": parity,
-            "shift_hints": "FP32 estimates for orders >= 48 (the default); the per-size plain launches use them "
-                           "for n >= 12"}
+            "arithmetic": "64-bit fixed point (the default), the capped per-size launches FP64"}
+
 
 def measure_reference_gpu(h, dev, stream, peak) -> dict:
     """The reference library itself (tokura_zgeev_batched_library, unmodified, built for sm_103a
@@ -976,6 +983,8 @@ def run_ours(args):
 
     kern_avg = statistics.mean(kern_ms)
     achieved = flops_per_matrix(N) * BATCH / (kern_avg * 1e-3)
+    int_peak = 2 * 32 / 3 * torch.cuda.get_device_properties(dev).multi_processor_count * 1e6 * (
+        clocks["sm_max_mhz"] if clocks else 2070)
     # DRAM bytes of one call: the per-matrix traffic of an ncu capture (profiles/traffic.json)
     # times this batch; the capture's conditions and the scaling are stated there.
     prof = read_profile_traffic()
@@ -984,9 +993,14 @@ def run_ours(args):
         traffic = prof["dram_bytes_per_matrix"] * BATCH
         traffic_note = prof.get("scaling")
     roofline = {
-        "bound": "fp64", "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": "TFLOP/s",
+        "bound": "fp64" if args.lanes else "integer multiplier (no FP64 in the main path: frac may pass 1)",
+        "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": "TFLOP/s",
         "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_note,
         "peak_source": "FP64 FMA-loop probe run in this process (MEASURED_PEAKS.json has no FP64 figure)",
+        # A product of 64-bit fixed point is three 32 x 32 + 64-bit multiply-adds, of which an SM issues
+        # 32 lanes a clock: 10.7 products a clock and SM.
+        "int_mad": {"peak": int_peak / 1e12, "unit": "TFLOP/s", "frac": achieved / int_peak,
+                    "peak_source": "32 multiply-adds a clock and SM (measured), 3 to a product, at the maximum clock"},
         "algorithmic": f"40*n^3 flops and 16*n^2+16*n+1 bytes per matrix x {BATCH} matrices per launch",
         "kernel_ms_avg": kern_avg,
     }
@@ -1180,10 +1194,11 @@ def run_ours(args):
                        "l2": f"inputs ({16 * N * N * BATCH / 2 ** 20:.0f} MiB) "
                              f"{'larger' if 16 * N * N * BATCH > 129 * 2 ** 20 else 'smaller'} than L2 (129 MB)",
                        "lanes_per_matrix": h.plain_config(N, BATCH)[0],
-                       "shift_hints": "FP32 estimator on a second stream beside the FP64 Hessenberg kernel, then "
-                                      "the FP64 QR kernel" if N >= SHIFT_HINT_MIN_N else "off (n < 12)"},
+                       "arithmetic": "FP64 (launch shape set)" if args.lanes else
+                                     "64-bit fixed point on the integer multiplier, FP64 for what that leaves; "
+                                     "errors against extended precision below the FP64 kernels'"},
             "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clocks,
-            "gpu_launches": args.steps * (3 if N >= SHIFT_HINT_MIN_N else 1), "flagged": flagged, "parity": parity, "sweep": sweep,
+            "gpu_launches": args.steps * launches_per_call(N, args.lanes), "flagged": flagged, "parity": parity, "sweep": sweep,
             "config1_n32_10000": config1, "ragged": ragged, "config4_backward": config4,
             "config5_ragged_gd_graph": config5, "real_dgeev_n64": real, "eigenvectors_n64": vectors,
             "reference_gpu": reference_gpu,

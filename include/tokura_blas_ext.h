@@ -35,7 +35,9 @@ TOKURA_API int tokuraSetSweepCap(tokurablas_t* handle, int cap);
  * gain accuracy. Returns 0, -1 NULL handle, -2 bad mode. */
 TOKURA_API int tokuraSetBalancing(tokurablas_t* handle, int mode);
 
-/* FP32 shift hints for later eigenvalue calls on this handle. A separate,
+/* FP32 shift hints for later eigenvalue calls on this handle; any call of this
+ * function also keeps them on the FP64 kernels (tokura_zgeev_batched_gpu_fp64
+ * below says what the default is). A separate,
  * cheap kernel (one warp per matrix in shared memory) computes
  * single-precision eigenvalue estimates, running on a second stream beside
  * the FP64 Hessenberg phase; the FP64 QR then uses the nearest unused
@@ -225,15 +227,17 @@ TOKURA_API int tokuraHostAlloc(void** ptr, size_t bytes);
 TOKURA_API int tokuraHostFree(void* ptr);
 
 /* Host-to-device rate (GB/s) that tokura_zgeev_batched_host plans its chunks
- * for; 0 (the default) uses the rate its previous call on the handle measured.
+ * for where they depend on it (see there); 0 (the default) uses the rate its
+ * previous call on the handle measured.
  * Returns 0; -1 NULL handle, -2 gbs negative or not finite. */
 TOKURA_API int tokuraSetHostLinkRate(tokurablas_t* handle, double gbs);
 
 /* Host-buffer variant of tokura_zgeev_batched_gpu: A, eigenvalues and flag are
  * HOST pointers (layouts as the device call). The batch is cut into chunks of
- * chunk_matrices (0 = automatic: 2 equal chunks, or growing chunks from 1/16
- * of the batch when the previous call on the handle saw a host-to-device rate
- * below 100 GB/s) issued round-robin on the handle's own streams, copies in
+ * chunk_matrices (0 = automatic: 1/8, 1/4, 1/4, 1/4, 1/8 of a batch of 192
+ * matrices per SM or more in fixed point, solved one after another; else 2 equal
+ * chunks, or growing chunks from 1/16 of the batch when the previous call on the
+ * handle saw a host-to-device rate below 100 GB/s) issued round-robin on the handle's own streams, copies in
  * chunk order, so host-device copies overlap the solves; returns when the results
  * are in host memory. Replaces the reference's multi-stream example driver
  * (stream_test_with_MKL/main.cu:236-288). Host memory should be pinned for the
@@ -286,9 +290,12 @@ TOKURA_API int tokura_cgeev_batched_gpu(tokurablas_t* handle, int n, int batch_c
  * column-major at A + j*n*n; eigenvalue i of matrix j is
  * wr[i + j*n] + i*wi[i + j*n], in LAPACK's convention: complex conjugate
  * pairs are adjacent with the positive imaginary part first and are exact
- * conjugates; real eigenvalues have wi exactly 0. Computed by a real
- * Householder Hessenberg reduction and the Francis double-shift QR in FP64
- * (about a quarter of the complex path's arithmetic). flag[j] as for
+ * conjugates; real eigenvalues have wi exactly 0. Orders of 3 and more are
+ * computed in 64-bit fixed point (a real Householder reduction, the complex QR,
+ * eigenvalues paired at the end); smaller orders, matrices that this leaves
+ * (graded, triangular, conjugates not clear) and calls on a handle with a launch
+ * shape or balancing by a real reduction and the Francis double-shift QR in
+ * FP64. flag[j] as for
  * tokura_zgeev_batched_gpu (balancing per tokuraSetBalancing, sweep cap per
  * tokuraSetSweepCap). work: tokura_get_dgeev_workspacesize(n, batch_count)
  * bytes. A is read only. Returns 0; -1 NULL handle, -2 bad n, -3 A NULL,

@@ -12,7 +12,9 @@
 // strided, pointer-array and single-precision batches all run this code, so
 // their results are bitwise equal on the same matrix entries.
 //
-// Without shift hints the solve is one kernel (phase kAll). With hints it is
+// With the library's choices (tokura_handle.h: use_fixed) the matrices are solved in 64-bit fixed point
+// (zgeev_fixed_launch.cuh) and the FP64 kernel below takes those which that leaves; the FP64 path alone is:
+// without shift hints the solve is one kernel (phase kAll). With hints it is
 // two kernels with the FP32 estimator beside the first:
 //   caller's stream: [kPrepare: stage + Hessenberg] --join--> [kQR: QR with hints]
 //   second stream:   [FP32 estimator] -----------------^
