@@ -1,0 +1,139 @@
+"""Matrices that fixed point leaves to the FP64 kernels because of their entries' sizes: every entry point
+gives the FP64 kernels' results for them, whatever else is in the batch."""
+import numpy as np
+import pytest
+
+from oracle import lapack_oracle as lo
+from tokura_zgeev_batched_gb300 import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+
+def bits(t):
+    import torch
+
+    a = t.detach()
+    a = torch.view_as_real(a) if a.is_complex() else a
+    return a.cpu().numpy().view(np.uint64)
+
+
+def fp64_handle():
+    from tokura_zgeev_batched_gb300 import api
+
+    h = api.Handle()
+    assert h.set_shift_hints(0) == 0  # the FP64 iteration without hints
+    return h
+
+
+def block_diagonal(seed, n, scale):
+    """diag(B, scale B'), with its blocks' spectra by LAPACK."""
+    A = np.zeros((n, n), dtype=np.complex128)
+    k = n // 2
+    A[:k, :k] = wl.gaussian(1, k, seed=seed)[0]
+    small = wl.gaussian(1, n - k, seed=seed + 1)[0]
+    A[k:, k:] = np.ldexp(small.view(np.float64), scale).view(np.complex128)
+    return A, [(A[:k, :k], 0), (small, scale)]
+
+
+def below_the_unit(n, seed, real=False):
+    """Graded ones at places 1, 4 and 6: a block, and one diagonal entry, below 2^-61 of the norm."""
+    A = wl.gaussian(9, n, seed=seed)
+    A[1], blocks = block_diagonal(seed + 10, n, -70)
+    A[4] = block_diagonal(seed + 20, n, -200)[0]
+    A[6, n - 1] = 0
+    A[6, :, n - 1] = 0
+    A[6, n - 1, n - 1] = 2.0 ** -90 * 3
+    return (np.ascontiguousarray(A.real) if real else A), blocks
+
+
+LEFT = [1, 4, 6]
+
+
+@pytest.mark.parametrize("n", [4, 7, 16, 20, 33, 64])
+def test_what_is_below_the_unit_is_not_lost(cuda, n):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A, blocks = below_the_unit(n, 6100 + n)
+    M = torch.from_numpy(A).cuda()
+    w, f = api.zgeev_batched(M)
+    w64, f64 = api.zgeev_batched(M, handle=fp64_handle())
+    assert np.array_equal(bits(w[LEFT]), bits(w64[LEFT])) and torch.equal(f[LEFT], f64[LEFT])
+    assert f[1] == 0 and f[6] == 0
+    assert float((w[6] - 3 * 2.0 ** -90).abs().min()) <= 3 * 2.0 ** -90 * 1e-14
+    # the small block's eigenvalues to the parity bound of its own norm
+    got = w[1].cpu().numpy()
+    got = got[np.argsort(np.abs(got))]
+    small, scale = blocks[1]
+    k = len(small)
+    ref = lo.zgeev(small[None])[0]
+    err = lo.matched_abs_errors(np.ldexp(got[:k].copy().view(np.float64), -scale).view(np.complex128)[None], ref)
+    assert err.max() <= lo.TOL_REL_FRO * np.linalg.norm(small)
+
+
+@pytest.mark.parametrize("n", [4, 7, 16, 20, 33, 64])
+def test_what_is_below_the_unit_is_not_lost_in_real_matrices(cuda, n):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A, _ = below_the_unit(n, 6200 + n, real=True)
+    M = torch.from_numpy(A).cuda()
+    h = api.Handle()
+    assert h.set_real_config(n, 8 if n >= 16 else 4, 32) == 0  # what so small a batch uses
+    for got, ref in zip(api.dgeev_batched(M), api.dgeev_batched(M, handle=h)):
+        assert torch.equal(got[LEFT], ref[LEFT])
+
+
+def packed(A):
+    import torch
+
+    ns = torch.full((len(A),), A.shape[1], dtype=torch.int32)
+    return torch.from_numpy(A).cuda().reshape(-1), ns
+
+
+@pytest.mark.parametrize("n", [4, 7, 16, 20, 33])
+def test_what_is_below_the_unit_is_not_lost_in_ragged_calls(cuda, n):
+    """Orders below those that the FP64 path has shift hints for."""
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A, _ = below_the_unit(n, 6300 + n)
+    buf, ns = packed(A)
+    w, f = api.zgeev_ragged(buf, ns)
+    w64, f64 = api.zgeev_ragged(buf, ns, handle=fp64_handle())
+    assert torch.equal(f, f64)
+    assert np.array_equal(bits(w.reshape(-1, n)[LEFT]), bits(w64.reshape(-1, n)[LEFT]))
+
+
+@pytest.mark.parametrize("n", [5, 7, 16, 20, 33, 64])
+def test_what_is_below_the_unit_is_not_lost_in_schur_forms(cuda, n):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A, blocks = below_the_unit(n, 6400 + n)
+    M = torch.from_numpy(A).cuda()
+    w, VL, VR, f = api.zgeev_vectors(M)
+    assert f[1] == 0
+    got = w[1].cpu().numpy()
+    got = got[np.argsort(np.abs(got))]
+    small, scale = blocks[1]
+    ref = lo.zgeev(small[None])[0]
+    k = len(small)
+    err = lo.matched_abs_errors(np.ldexp(got[:k].copy().view(np.float64), -scale).view(np.complex128)[None], ref)
+    assert err.max() <= lo.TOL_REL_FRO * np.linalg.norm(small)
+    # gradients: the FP64 kernel's, from the same eigenvalues
+    lam, _ = api.zgeev_batched(M, handle=fp64_handle())
+    gbar = (torch.exp(lam.real) + 2 * lam).contiguous()
+    out = []
+    for h in (api.default_handle(), fp64_handle()):
+        ns = torch.full((len(A),), n, dtype=torch.int32, device="cuda")
+        offs = torch.arange(len(A), dtype=torch.int64, device="cuda") * (n * n)
+        work = torch.empty(api.tokura_get_zgeev_ragged_backward_workspacesize(len(A), M.numel()), dtype=torch.uint8,
+                           device="cuda")
+        g, flag = torch.empty_like(M), torch.empty(len(A), dtype=torch.int8, device="cuda")
+        assert api.tokura_zgeev_ragged_backward_gpu(h, len(A), ns.data_ptr(), offs.data_ptr(), None, M.numel(),
+                                                    M.data_ptr(), lam.data_ptr(), gbar.data_ptr(), g.data_ptr(),
+                                                    work.data_ptr(), flag.data_ptr(),
+                                                    torch.cuda.current_stream().cuda_stream) == 0
+        out.append((bits(g[LEFT]), flag[LEFT].cpu()))
+    assert np.array_equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])

@@ -102,6 +102,8 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) real_hess_kernel(int n, int b
       if (G.rank == 0) flag[j] = (char)(emax != 0 ? kNonFinite : kConverged);
     } else {
       G.sync();
+      const bool left = left_to_fp64(G, n, emax, [&](int r, int c) { return magnitude_bits(A[c * ld + r]); });
+      G.sync();
       float s2 = 0.0f;
       for (int c = G.rank; c < n; c += L)
         for (int r = 0; r < n; ++r) {
@@ -109,31 +111,18 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) real_hess_kernel(int n, int b
           s2 = fmaf(x, x, s2);
         }
       const int p = exponent_of(kFixedNormMax / mulf(sqrtf(G.sumf(s2)), 1.0001f));
-      unsigned long long lower = 0, upper = 0, all = 0, least = ~0ull;  // as for complex matrices
-      for (int c = G.rank; c < n; c += L) {
-        unsigned long long column = 0;
+      unsigned long long lower = 0, upper = 0;  // as for complex matrices
+      for (int c = G.rank; c < n; c += L)
         for (int r = 0; r < n; ++r) {
           const long long w = to_fixed(A[c * ld + r], emax, p);
           A[c * ld + r] = w;
           const unsigned long long v = mag64(w - kZero);
-          column |= v;
           if (r > c) lower |= v;
           if (r < c) upper |= v;
         }
-        all |= column;
-        if (column != 0 && column < least) least = column;
-      }
-      G.sync();
-      for (int r = G.rank; r < n; r += L) {
-        unsigned long long row = 0;
-        for (int c = 0; c < n; ++c) row |= mag64(A[c * ld + r] - kZero);
-        if (row != 0 && row < least) least = row;
-      }
-      all = G.ior(all);
       lower = G.ior(lower);
       upper = G.ior(upper);
-      const int spread = G.imax(clz64(least)) - clz64(all);
-      st = lower == 0 || upper == 0 || spread > kFixedGradedBits ? kStateGeneral : emax - 1023 - p;
+      st = left || lower == 0 || upper == 0 ? kStateGeneral : emax - 1023 - p;
     }
     if (G.rank == 0) {
       work[(j + 1) * real_words(n) - 1] = st == kStateGeneral ? kStateDone : st;

@@ -16,13 +16,10 @@
 #pragma once
 
 #include "zgeev_fixed.cuh"
+#include "zgeev_fixed_guard.cuh"
 #include "zgeev_fixed_qr.cuh"
 
 namespace tzg {
-
-// A row or column whose largest entry is this many binades below the matrix's largest
-// makes the matrix a graded one, which the FP64 kernels solve.
-constexpr int kFixedGradedBits = 12;
 
 template <int L>
 inline size_t fixed_hess_shared(int n) {
@@ -33,6 +30,7 @@ inline size_t fixed_hess_shared(int n) {
 // Lane group of a warp part or a whole block.
 template <int L>
 struct FixedGroup {
+  static constexpr int kLanes = L;
   int rank;
   unsigned mask;
   unsigned long long* scratch;  // 32 words shared by the block's warps (L > 32)
@@ -315,6 +313,11 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
         if (G.rank == 0) flag[j] = (char)(emax != 0 ? kNonFinite : kConverged);
       } else {
         G.sync();
+        const bool left = left_to_fp64(G, n, emax, [&](int r, int c) {
+          const cfx z = A[c * ld + r];
+          return max(magnitude_bits(z.x), magnitude_bits(z.y));
+        });
+        G.sync();
         float s2 = 0.0f;
         for (int c = G.rank; c < n; c += L)
           for (int r = 0; r < n; ++r) {
@@ -323,34 +326,21 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
           }
         const float top = kFixedNormMax / mulf(sqrtf(G.sumf(s2)), 1.0001f);
         const int p = exponent_of(top);
-        // Fixed point. Matrices with a row or column whose largest entry is far below the matrix's, and triangular
-        // ones (an upper triangular one's diagonal is exact in FP64), are left to the FP64 kernels.
-        unsigned long long lower = 0, upper = 0, all = 0, least = ~0ull;
-        for (int c = G.rank; c < n; c += L) {
-          unsigned long long column = 0;
+        // Fixed point. Triangular matrices are left to the FP64 kernels too (an upper triangular one's diagonal is
+        // exact there).
+        unsigned long long lower = 0, upper = 0;
+        for (int c = G.rank; c < n; c += L)
           for (int r = 0; r < n; ++r) {
             const cfx z = A[c * ld + r];
             const cfx w = {to_fixed(z.x, emax, p), to_fixed(z.y, emax, p)};
             A[c * ld + r] = w;
             const unsigned long long v = mag64(w.x - kZero) | mag64(w.y - kZero);
-            column |= v;
             if (r > c) lower |= v;
             if (r < c) upper |= v;
           }
-          all |= column;
-          if (column != 0 && column < least) least = column;
-        }
-        G.sync();
-        for (int r = G.rank; r < n; r += L) {
-          unsigned long long row = 0;
-          for (int c = 0; c < n; ++c) row |= mag64(A[c * ld + r].x - kZero) | mag64(A[c * ld + r].y - kZero);
-          if (row != 0 && row < least) least = row;
-        }
-        all = G.ior(all);
         lower = G.ior(lower);
         upper = G.ior(upper);
-        const int spread = G.imax(clz64(least)) - clz64(all);
-        st = lower == 0 || upper == 0 || spread > kFixedGradedBits ? kStateGeneral : emax - 1023 - p;
+        st = left || lower == 0 || upper == 0 ? kStateGeneral : emax - 1023 - p;
       }
     }
     if (G.rank == 0) *(kQ ? schur_state(hess + tile.where + (long long)slot * nn, n) : state + j) = st;
