@@ -65,7 +65,9 @@ def rule(A):
     e = exponents(A)
     top = e.max((1, 2))[:, None]
     row, column = e.max(2), e.max(1)
-    return ((row > NONE) & (top - row > 12)).any(1) | ((column > NONE) & (top - column > 12)).any(1)
+    both = np.maximum(row, column)
+    return (((row > NONE) & (top - row > 8)) | ((column > NONE) & (top - column > 12)) |
+            ((both > NONE) & (top - both > 5))).any(1)
 
 
 def graded(n, seed):
@@ -74,7 +76,7 @@ def graded(n, seed):
     A = wl.gaussian(600, n, seed=seed)
     for M in A:
         for _ in range(rng.integers(0, 3)):
-            i, s = rng.integers(n), 2.0 ** -float(rng.choice([3, 6, 10, 12, 13, 30, 61, 62, 200, 1000, 1070]))
+            i, s = rng.integers(n), 2.0 ** -float(rng.choice([3, 5, 6, 8, 9, 12, 13, 30, 61, 62, 200, 1000, 1070]))
             kind = rng.integers(4)
             if kind in (0, 2):
                 M[i] *= s

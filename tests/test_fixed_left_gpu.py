@@ -137,3 +137,39 @@ def test_what_is_below_the_unit_is_not_lost_in_schur_forms(cuda, n):
                                                     torch.cuda.current_stream().cuda_stream) == 0
         out.append((bits(g[LEFT]), flag[LEFT].cpu()))
     assert np.array_equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+def graded_a_little(n, seed, real=False):
+    """Matrices whose small eigenvalues FP64 holds to their relative precision and an absolute unit does not."""
+    A = wl.gaussian(12, n, seed=seed)
+    k = n // 2
+    down = 2.0 ** np.linspace(0, -9, n)
+    for j, s in ((1, 7), (2, 11)):  # two blocks
+        A[j, :k, k:] = 0
+        A[j, k:, :k] = 0
+        A[j, k:, k:] = np.ldexp(A[j, k:, k:].copy().view(np.float64), -s).view(np.complex128)
+    A[4] *= down[:, None] * down  # rows and columns
+    A[5, n - 1] *= 2.0 ** -8  # one row and column
+    A[5, :, n - 1] *= 2.0 ** -8
+    A[7] *= 2.0 ** np.linspace(0, -12, n)  # rows (of the column-major matrix)
+    return np.ascontiguousarray(A.real) if real else A
+
+
+GRADED = [1, 2, 4, 5, 7]
+
+
+@pytest.mark.parametrize("n", [2, 4, 9, 20, 50])
+def test_slightly_graded_matrices_are_left_to_fp64(cuda, n):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    M = torch.from_numpy(graded_a_little(n, 6500 + n)).cuda()
+    w, f = api.zgeev_batched(M)
+    w64, f64 = api.zgeev_batched(M, handle=fp64_handle())
+    assert np.array_equal(bits(w[GRADED]), bits(w64[GRADED])) and torch.equal(f, f64)
+    if n > 2:
+        R = torch.from_numpy(graded_a_little(n, 6500 + n, real=True)).cuda()
+        h = api.Handle()
+        assert h.set_real_config(n, 8 if n >= 16 else 4, 32) == 0
+        for got, ref in zip(api.dgeev_batched(R), api.dgeev_batched(R, handle=h)):
+            assert torch.equal(got[GRADED], ref[GRADED])
