@@ -18,20 +18,24 @@ using namespace tzg;
 struct OneLane {
   static constexpr int kLanes = 1;
   int rank = 0;
+  void sync() const {}
   unsigned long long ior(unsigned long long v) const { return v; }
+  int imax(int v) const { return v; }
 };
 // Column-major n x n complex matrices.
 extern "C" void left(const long long* a, int n, int batch, int* out) {
+  int scale[128];
   for (int j = 0; j < batch; ++j, a += 2 * n * n) {
     int emax = 0;
     for (int e = 0; e < 2 * n * n; ++e) {
-      const int x = (int)(magnitude_bits(a[e]) >> 52);
+      const int x = (int)(size_of(a[e]) >> 20);
       emax = x > emax ? x : emax;
     }
-    out[j] = emax != 0 && left_to_fp64(OneLane(), n, emax, [&](int r, int c) {  // subnormal ones: not asked
-      const unsigned long long x = magnitude_bits(a[2 * (c * n + r)]), y = magnitude_bits(a[2 * (c * n + r) + 1]);
+    const auto size = [&](int r, int c) {
+      const unsigned x = size_of(a[2 * (c * n + r)]), y = size_of(a[2 * (c * n + r) + 1]);
       return x > y ? x : y;
-    });
+    };
+    out[j] = emax != 0 && left_to_fp64(OneLane(), n, emax, size, size, scale);  // subnormal ones: not asked
   }
 }
 """
@@ -67,7 +71,28 @@ def rule(A):
     row, column = e.max(2), e.max(1)
     both = np.maximum(row, column)
     return (((row > NONE) & (top - row > 8)) | ((column > NONE) & (top - column > 12)) |
-            ((both > NONE) & (top - both > 5))).any(1)
+            ((both > NONE) & (top - both > 5))).any(1) | unbalanced(e)
+
+
+def unbalanced(e):
+    """The span of the scales that balance a matrix, in eighths of a binade, all indices at once."""
+    n = e.shape[1]
+    off = np.where(e > NONE, 8 * e, 8 * NONE)
+    off[:, np.arange(n), np.arange(n)] = 8 * NONE
+    s = np.zeros(e.shape[:2], dtype=np.int64)
+    found = np.zeros(len(e), dtype=bool)
+    live = None
+    for step in range(16):
+        row, column = (off + s[:, None, :]).max(2), (off - s[:, :, None]).max(1)
+        d = np.where((row > 4 * NONE) & (column > 4 * NONE), row - column - 2 * s, 0)
+        if live is None:
+            live = (d.max(1) >= 24) & (d.min(1) <= -24)
+        live = live & (np.abs(d).max(1) >= 4)
+        s = s + np.where(live[:, None], np.sign(d) * (np.abs(d) // 2), 0)
+        span = s.max(1) - s.min(1)
+        found |= live & (span >= 64)
+        live = live & ~found & (span >= (32 if step >= 2 else 0))
+    return found
 
 
 def graded(n, seed):
@@ -95,6 +120,41 @@ def test_the_rule(left, n):
     want = rule(A)
     assert want.any() and not want.all()
     assert np.array_equal(left(A), want)
+
+
+def scaled(n, seed):
+    """D^-1 B D for tridiagonal, Hessenberg and dense B and all kinds of D."""
+    rng = np.random.default_rng(seed)
+    A = wl.gaussian(400, n, seed=seed)
+    for j, M in enumerate(A):
+        if j % 3 == 0:
+            M *= np.tri(n, n, 1) * np.tri(n, n, 1).T
+        elif j % 3 == 1:
+            M *= np.tri(n, n, 1).T
+        k = float(rng.choice([0, 1, 2, 3, 4, 6, 9])) / (1 if j % 3 == 0 else max(1, n - 1))
+        d = 2.0 ** (k * np.arange(n))
+        d = d if j % 2 else d[rng.permutation(n)]
+        M *= d / d[:, None]
+    return A
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 9, 33, 64])
+def test_the_rule_on_badly_balanced_matrices(left, n):
+    A = scaled(n, 6020 + n)
+    want = rule(A)
+    assert want.any() and not want.all()
+    assert np.array_equal(left(A), want)
+    # the scales alone
+    only = [j for j in range(len(A)) if unbalanced(exponents(A[j:j + 1]))[0]]
+    assert len(only) >= 20
+
+
+@pytest.mark.parametrize("n,k,is_left", [(3, 2, False), (8, 1, False), (64, 1, False), (6, 2, True), (12, 2, True),
+                                         (6, 3, True), (12, 3, True), (4, 4, True), (64, 3, True), (4, 8, True)])
+def test_scaled_toeplitz_matrices(left, n, k, is_left):
+    A = np.diag(np.full(n - 1, 2.0 ** k), 1) + np.diag(np.full(n - 1, 2.0 ** -k), -1) + np.eye(n)
+    both = np.stack([A, A.T]).astype(np.complex128)
+    assert (left(both) == is_left).all() and (rule(both) == is_left).all()
 
 
 def test_what_is_below_the_unit_counts(left):

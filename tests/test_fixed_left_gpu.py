@@ -173,3 +173,37 @@ def test_slightly_graded_matrices_are_left_to_fp64(cuda, n):
         assert h.set_real_config(n, 8 if n >= 16 else 4, 32) == 0
         for got, ref in zip(api.dgeev_batched(R), api.dgeev_batched(R, handle=h)):
             assert torch.equal(got[GRADED], ref[GRADED])
+
+
+def badly_balanced(n, seed, real=False):
+    """Tridiagonal ones 2^k, 1, 2^-k (places 0 and 1, spectra known) and D^-1 B D."""
+    A = np.empty((5, n, n), dtype=np.complex128)
+    for j, k in ((0, 4), (1, 8)):
+        A[j] = np.diag(np.full(n - 1, 2.0 ** k), 1) + np.diag(np.full(n - 1, 2.0 ** -k), -1) + np.eye(n)
+    d = 2.0 ** np.linspace(0, 11, n)
+    A[2:] = wl.gaussian(3, n, seed=seed) * d / d[:, None]
+    A[3] = np.swapaxes(A[3], 0, 1)
+    if real:
+        A = A.real + A.imag
+    return np.ascontiguousarray(A)
+
+
+@pytest.mark.parametrize("n", [4, 6, 16, 33, 64])
+def test_badly_balanced_matrices_are_left_to_fp64(cuda, n):
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    A = badly_balanced(n, 6600 + n)
+    M = torch.from_numpy(A).cuda()
+    w, f = api.zgeev_batched(M)
+    w64, f64 = api.zgeev_batched(M, handle=fp64_handle())
+    assert np.array_equal(bits(w), bits(w64)) and torch.equal(f, f64)
+    if n <= 6:  # (above, FP64 without balancing does not hold them either)
+        exact = 1 + 2 * np.cos(np.arange(1, n + 1) * np.pi / (n + 1))
+        err = lo.matched_abs_errors(w[:2].cpu().numpy(), np.stack([exact, exact]).astype(np.complex128))
+        assert err.max() <= lo.TOL_REL_FRO * np.linalg.norm(A[0])
+    R = torch.from_numpy(badly_balanced(n, 6600 + n, real=True)).cuda()
+    h = api.Handle()
+    assert h.set_real_config(n, 8 if n >= 16 else 4, 32) == 0
+    for got, ref in zip(api.dgeev_batched(R), api.dgeev_batched(R, handle=h)):
+        assert torch.equal(got, ref)

@@ -19,31 +19,96 @@ constexpr int kFixedGradedRow = 8;
 constexpr int kFixedGradedColumn = 12;
 constexpr int kFixedGradedIndex = 5;
 
-// floor(log2 |x|) + 1023 from the bits of |x|, subnormal numbers among them.
-TZG_HD int bits_exponent(unsigned long long magnitude) {
-  const int e = (int)(magnitude >> 52);
-  return e != 0 ? e : 12 - clz64(magnitude);
-}
-TZG_HD unsigned long long magnitude_bits(long long bits) { return (unsigned long long)bits & 0x7fffffffffffffffull; }
+// Badly balanced matrices, D^-1 B D: their eigenvalues are as ill-conditioned normwise as D is, but FP64 keeps those of
+// banded and Hessenberg ones all the same, having no absolute unit. A matrix is left if the scales that balance it (the
+// largest entries beside the diagonal of row i and column i alike) span this many binades. Errors over the norm, FP64 and
+// fixed point, tridiagonal 2^k, 1, 2^-k: k = 1, n = 24 7e-12 and 1e-12; k = 2, n = 12 9e-14 and 1e-13, n = 24 7e-9 and
+// 1e-6; k = 3, n = 3 4e-17 and 0, n = 6 4e-16 and 2e-15, n = 12 1e-13 and 2e-10; k = 10, n = 4 1e-18 and 1e-10. Relative
+// errors of dense ones, D = 1 .. 2^k: k = 6 1e-14 and 2e-14, k = 8 2e-14 and 3e-13. The scales are found in steps, all
+// indices at once, in parts of a binade; those of the matrices above span 4 binades in the third step, or never 8, and 8 in
+// the 13th at the latest. The search starts when one index's row and another's column are larger by three binades: in 1 of
+// 10,000 Gaussian matrices of order 4, 2 to 11 % of V diag V^-1 ones.
+constexpr int kFixedUnbalancedBits = 8;
+constexpr int kBalanceStart = 3;
+constexpr int kBalanceParts = 8;
+constexpr int kBalanceSteps = 16;
 
-// `top(r, c)`: magnitude_bits of the larger component of an entry; `emax`: the largest exponent field. The lanes of
-// `G` take the indices i (row i and column i) in turn; all of them get the answer.
-template <class Group, class Top>
-TZG_HD bool left_to_fp64(const Group& G, int n, int emax, Top top) {
-  bool graded = false;
+// The size of a number, from its bits: the high word of |x|, with a bit for what is below it (subnormal numbers count,
+// if only as far below all others). Then floor(log2 |x|) + 1023 of a size that is not 0.
+TZG_HD unsigned size_of(long long bits) {
+  return ((unsigned)(bits >> 32) & 0x7fffffffu) | ((unsigned)bits != 0 ? 1u : 0u);
+}
+TZG_HD int size_exponent(unsigned size) {
+  const int e = (int)(size >> 20);
+  return e != 0 ? e : 12 - clz32(size);
+}
+
+// `top(r, c)`: the larger component's size of an entry; `first(r, c)`: the same, called once for each entry before any
+// top (so that a caller can do more with it); `emax`: the largest exponent field; `scale`: 2n words that the lanes of `G`
+// share. The lanes take the indices i (row i and column i) in turn; all get the answer.
+template <class Group, class First, class Top>
+TZG_HD bool left_to_fp64(const Group& G, int n, int emax, First first, Top top, int* scale) {
+  bool graded = false, up = false, down = false;
   for (int i = G.rank; i < n; i += Group::kLanes) {
-    unsigned long long row = 0, column = 0;
+    unsigned row = 0, column = 0, diagonal = 0;
     for (int k = 0; k < n; ++k) {
-      const unsigned long long a = top(i, k), b = top(k, i);
-      row = a > row ? a : row;
-      column = b > column ? b : column;
+      const unsigned b = first(k, i);
+      if (k == i)
+        diagonal = b;
+      else
+        column = b > column ? b : column;
     }
-    const unsigned long long both = row > column ? row : column;
-    graded |= row != 0 && emax - bits_exponent(row) > kFixedGradedRow;
-    graded |= column != 0 && emax - bits_exponent(column) > kFixedGradedColumn;
-    graded |= both != 0 && emax - bits_exponent(both) > kFixedGradedIndex;
+    for (int k = 0; k < n; ++k) {
+      const unsigned a = k != i ? top(i, k) : 0u;
+      row = a > row ? a : row;
+    }
+    if (row != 0 && column != 0) {
+      const int d = size_exponent(row) - size_exponent(column);
+      up |= d >= kBalanceStart;
+      down |= d <= -kBalanceStart;
+    }
+    row = diagonal > row ? diagonal : row;
+    column = diagonal > column ? diagonal : column;
+    const unsigned both = row > column ? row : column;
+    graded |= row != 0 && emax - size_exponent(row) > kFixedGradedRow;
+    graded |= column != 0 && emax - size_exponent(column) > kFixedGradedColumn;
+    graded |= both != 0 && emax - size_exponent(both) > kFixedGradedIndex;
   }
-  return G.ior(graded) != 0;
+  const unsigned long long found = G.ior((graded ? 1u : 0u) | (up ? 2u : 0u) | (down ? 4u : 0u));
+  if (found & 1) return true;
+  if (found != 6) return false;
+  constexpr int kNone = -(1 << 28), kBias = 1 << 24;  // scales stay far below the bias
+  int *now = scale, *next = scale + n;
+  for (int i = G.rank; i < n; i += Group::kLanes) now[i] = 0;
+  for (int step = 0; step < kBalanceSteps; ++step) {
+    G.sync();
+    int low = kBias, high = -kBias;
+    bool moving = false;
+    for (int i = G.rank; i < n; i += Group::kLanes) {
+      int row = kNone, column = kNone;
+      for (int k = 0; k < n; ++k) {
+        if (k == i) continue;
+        const unsigned a = top(i, k), b = top(k, i);
+        const int r = kBalanceParts * size_exponent(a) + now[k], c = kBalanceParts * size_exponent(b) - now[k];
+        if (a != 0 && r > row) row = r;
+        if (b != 0 && c > column) column = c;
+      }
+      const int d = row > kNone && column > kNone ? row - column - 2 * now[i] : 0;
+      moving |= d >= kBalanceParts / 2 || d <= -kBalanceParts / 2;
+      const int v = now[i] + d / 2;
+      next[i] = v;
+      low = v < low ? v : low;
+      high = v > high ? v : high;
+    }
+    if (!G.ior(moving)) return false;
+    const int span = G.imax(high + kBias) + G.imax(kBias - low) - 2 * kBias;
+    if (span >= kFixedUnbalancedBits * kBalanceParts) return true;
+    if (step >= 2 && span < kFixedUnbalancedBits / 2 * kBalanceParts) return false;
+    int* const t = now;
+    now = next;
+    next = t;
+  }
+  return false;
 }
 
 }  // namespace tzg

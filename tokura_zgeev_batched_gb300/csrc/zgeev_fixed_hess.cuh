@@ -313,17 +313,18 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
         if (G.rank == 0) flag[j] = (char)(emax != 0 ? kNonFinite : kConverged);
       } else {
         G.sync();
+        float s2 = 0.0f;
+        const auto size = [&](int r, int c) {
+          const cfx z = A[c * ld + r];
+          return max(size_of(z.x), size_of(z.y));
+        };
         const bool left = left_to_fp64(G, n, emax, [&](int r, int c) {
           const cfx z = A[c * ld + r];
-          return max(magnitude_bits(z.x), magnitude_bits(z.y));
-        });
+          const float x = scaled_float(z.x, emax), y = scaled_float(z.y, emax);
+          s2 = fmaf(x, x, fmaf(y, y, s2));
+          return max(size_of(z.x), size_of(z.y));
+        }, size, reinterpret_cast<int*>(U));
         G.sync();
-        float s2 = 0.0f;
-        for (int c = G.rank; c < n; c += L)
-          for (int r = 0; r < n; ++r) {
-            const float x = scaled_float(A[c * ld + r].x, emax), y = scaled_float(A[c * ld + r].y, emax);
-            s2 = fmaf(x, x, fmaf(y, y, s2));
-          }
         const float top = kFixedNormMax / mulf(sqrtf(G.sumf(s2)), 1.0001f);
         const int p = exponent_of(top);
         // Fixed point. Triangular matrices are left to the FP64 kernels too (an upper triangular one's diagonal is
@@ -338,9 +339,8 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
             if (r > c) lower |= v;
             if (r < c) upper |= v;
           }
-        lower = G.ior(lower);
-        upper = G.ior(upper);
-        st = left || lower == 0 || upper == 0 ? kStateGeneral : emax - 1023 - p;
+        const bool full = G.ior((lower != 0 ? 1u : 0u) | (upper != 0 ? 2u : 0u)) == 3;
+        st = left || !full ? kStateGeneral : emax - 1023 - p;
       }
     }
     if (G.rank == 0) *(kQ ? schur_state(hess + tile.where + (long long)slot * nn, n) : state + j) = st;
