@@ -1,0 +1,132 @@
+"""Launch errors on the host, without a GPU: the library's own object files against a stand-in for the CUDA runtime that
+counts launches, fails the one it is told to, and writes down what reaches which stream. Work that was forked to the
+handle's second stream is joined again whatever fails after it."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "tokura_zgeev_batched_gb300")
+
+# The host side that nvcc generates calls the functions with two underscores.
+RUNTIME = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+#include <vector>
+#include <cuda_runtime.h>
+int launches = 0, fail_at = -1;
+cudaError_t last = cudaSuccess;
+std::string events;
+static void note(const char* what, cudaStream_t s) {
+  events += what;
+  events += s == (cudaStream_t)2 ? "2 " : "1 ";
+}
+static std::vector<std::pair<dim3, std::pair<dim3, std::pair<size_t, cudaStream_t>>>> pushed;
+extern "C" {
+void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterFunction(void**, const char*, char*, const char*, int, uint3*, uint3*, dim3*, dim3*, int*) {}
+void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
+cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* f) { *k = (cudaKernel_t)f; return cudaSuccess; }
+unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t m, cudaStream_t s) {
+  pushed.push_back({g, {b, {m, s}}});
+  return 0;
+}
+cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* m, void* s) {
+  *g = pushed.back().first;
+  *b = pushed.back().second.first;
+  *m = pushed.back().second.second.first;
+  *(cudaStream_t*)s = pushed.back().second.second.second;
+  pushed.pop_back();
+  return cudaSuccess;
+}
+cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void**, size_t, cudaStream_t s) {
+  if (launches++ == fail_at) {
+    note("failed", s);
+    return last = cudaErrorInvalidValue;
+  }
+  note("launch", s);
+  return cudaSuccess;
+}
+cudaError_t cudaGetLastError() { const cudaError_t e = last; last = cudaSuccess; return e; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  note(e == (cudaEvent_t)11 ? "fork" : "join", s);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
+  note(e == (cudaEvent_t)11 ? "afterfork" : "afterjoin", s);
+  return cudaSuccess;
+}
+cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 152; return cudaSuccess; }
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* b, const void*, int, size_t, unsigned) {
+  *b = 4;
+  return cudaSuccess;
+}
+}
+"""
+
+VECTORS = RUNTIME + r"""
+#include <mutex>
+#include "zgeev_internal.h"
+namespace tzg {
+size_t backward_workspace_bytes(int n, int batch) { return 64ull * n * n * batch; }
+}
+int main(int argc, char** argv) {
+  fail_at = std::atoi(argv[1]);
+  std::mutex mu;
+  tzg::ForkJoin fj;
+  fj.aux = (cudaStream_t)2;
+  fj.fork = (cudaEvent_t)11;
+  fj.join = (cudaEvent_t)12;
+  fj.mu = &mu;
+  double2* p = (double2*)4096;  // never read
+  const cudaError_t e = tzg::launch_vectors(4, std::atoi(argv[2]), 100, p, p, p, p, p, (char*)p, 300, (cudaStream_t)1,
+                                            true, &fj, 65, true);
+  std::printf("%d %s\n", (int)e, events.c_str());
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def vectors(tmp_path_factory):
+    sys.path.insert(0, ROOT)
+    from tokura_zgeev_batched_gb300 import build
+
+    build.build()
+    obj = os.path.join(PKG, "_build", "zgeev_vectors.cu.o")
+    if not os.path.exists(obj):
+        build.build(force=True)
+    d = tmp_path_factory.mktemp("launch")
+    (d / "vectors.cpp").write_text(VECTORS)
+    include = os.path.join(os.path.dirname(os.path.dirname(build._nvcc())), "include")
+    exe = str(d / "vectors")
+    subprocess.check_call(["g++", "-std=c++17", "-I", include, "-I", os.path.join(PKG, "csrc"), str(d / "vectors.cpp"),
+                           obj, "-o", exe, "-pthread"])
+
+    def run(fail_at, n):
+        out = subprocess.run([exe, str(fail_at), str(n)], capture_output=True, text=True, timeout=60, check=True).stdout
+        err, *events = out.split()
+        return int(err), events
+    return run
+
+
+@pytest.mark.parametrize("n", [12, 24, 40])
+def test_vectors_join_the_second_stream_after_a_failed_launch(vectors, n):
+    err, events = vectors(-1, n)
+    assert err == 0 and events.count("afterjoin1") == 1
+    launches = sum(e.startswith("launch") for e in events)
+    assert launches >= 4
+    for k in range(launches):
+        err, events = vectors(k, n)
+        assert err == 1, (k, events)
+        assert sum(e.startswith("failed") for e in events) == 1
+        fork, join, wait = (events.index(e) if e in events else -1 for e in ("afterfork2", "join2", "afterjoin1"))
+        assert fork >= 0 and fork < join < wait, (k, events)
+        assert not any(e.endswith("2") for e in events[join + 1:]), (k, events)

@@ -222,11 +222,15 @@ cudaError_t launch_vectors(int lanes, int n, int batch, const double2* A, double
       lock = std::unique_lock<std::mutex>(*fj->mu);
       if ((err = cudaEventRecord(fj->fork, stream)) != cudaSuccess) return err;
       if ((err = cudaStreamWaitEvent(fj->aux, fj->fork, 0)) != cudaSuccess) return err;
-      if ((err = launch_estimates(n, batch, src, est, fj->aux)) != cudaSuccess) return err;
-      if ((err = cudaEventRecord(fj->join, fj->aux)) != cudaSuccess) return err;
+      err = launch_estimates(n, batch, src, est, fj->aux);
     }
-    if ((err = launch_schur_hess(list, n, batch, src, hess, q, 0, stream)) != cudaSuccess) return err;
-    if (beside && (err = cudaStreamWaitEvent(stream, fj->join, 0)) != cudaSuccess) return err;
+    if (err == cudaSuccess) err = launch_schur_hess(list, n, batch, src, hess, q, 0, stream);
+    if (beside) {  // also after a failed launch: the second stream rejoins the caller's
+      const cudaError_t e1 = cudaEventRecord(fj->join, fj->aux);
+      const cudaError_t e2 = cudaStreamWaitEvent(stream, fj->join, 0);
+      if (err == cudaSuccess) err = e1 != cudaSuccess ? e1 : e2;
+    }
+    if (err != cudaSuccess) return err;
     const SchurDone done{work, nullptr, nullptr, nullptr, w, flag};
     if ((err = launch_schur_qr(list, n, batch, EstimateShifts{est}, done, hess, q, itmax, 1, 0, stream)) !=
         cudaSuccess)
