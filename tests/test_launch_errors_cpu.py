@@ -93,22 +93,64 @@ int main(int argc, char** argv) {
 }
 """
 
+TUNER = RUNTIME + r"""
+#include "tokura_handle.h"
+#include "tokura_blas_ext.h"
+static int calls = 0;
+static cudaError_t timed() { return calls++ == fail_at ? cudaErrorUnknown : cudaSuccess; }
+namespace tzg {
+cudaError_t launch_plain(const PlainConfig&, int, int, const double2*, double2*, double2*, char*, int, cudaStream_t, int,
+                         bool, const ForkJoin*) {
+  return timed();
+}
+cudaError_t launch_ragged(int, int, int, const int*, const long long*, const long long*, long long, const double2*,
+                          double2*, void*, char*, int, cudaStream_t, int, int, const ForkJoin*, int, bool) {
+  return timed();
+}
+size_t ragged_workspace_bytes(int, long long) { return 256; }
+}
+extern "C" {
+cudaError_t cudaMalloc(void** p, size_t) { *p = (void*)4096; return cudaSuccess; }
+cudaError_t cudaFree(void*) { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)12; return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 100.0f - calls; return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGetDeviceProperties(cudaDeviceProp*, int) { return cudaErrorUnknown; }
+}
+int main(int argc, char** argv) {
+  fail_at = std::atoi(argv[1]);
+  tokurablas_t h;
+  h.sm_count = 152;
+  h.plain[20] = tzg::PlainConfig{4, 64};
+  h.ragged_lanes = 2;
+  const int st = argv[2][0] == 'p' ? tokuraAutotune(&h, 20, 20, 100, 0) : tokuraAutotuneRagged(&h, 100, 2, 20, 0);
+  std::printf("%d %d %d %d %d\n", st, calls, h.plain[20].lanes, h.plain[20].threads, h.ragged_lanes);
+}
+"""
 
-@pytest.fixture(scope="module")
-def vectors(tmp_path_factory):
+
+def linked(source, name, directory):
+    """`source` with the library's object file of that translation unit."""
     sys.path.insert(0, ROOT)
     from tokura_zgeev_batched_gb300 import build
 
     build.build()
-    obj = os.path.join(PKG, "_build", "zgeev_vectors.cu.o")
+    obj = os.path.join(PKG, "_build", name + ".o")
     if not os.path.exists(obj):
         build.build(force=True)
-    d = tmp_path_factory.mktemp("launch")
-    (d / "vectors.cpp").write_text(VECTORS)
+    (directory / "main.cpp").write_text(source)
     include = os.path.join(os.path.dirname(os.path.dirname(build._nvcc())), "include")
-    exe = str(d / "vectors")
-    subprocess.check_call(["g++", "-std=c++17", "-I", include, "-I", os.path.join(PKG, "csrc"), str(d / "vectors.cpp"),
-                           obj, "-o", exe, "-pthread"])
+    exe = str(directory / "main")
+    subprocess.check_call(["g++", "-std=c++17", "-I", include, "-I", os.path.join(PKG, "csrc"), "-I",
+                           os.path.join(ROOT, "include"), str(directory / "main.cpp"), obj, "-o", exe, "-pthread"])
+    return exe
+
+
+@pytest.fixture(scope="module")
+def vectors(tmp_path_factory):
+    exe = linked(VECTORS, "zgeev_vectors.cu", tmp_path_factory.mktemp("vectors"))
 
     def run(fail_at, n):
         out = subprocess.run([exe, str(fail_at), str(n)], capture_output=True, text=True, timeout=60, check=True).stdout
@@ -130,3 +172,22 @@ def test_vectors_join_the_second_stream_after_a_failed_launch(vectors, n):
         fork, join, wait = (events.index(e) if e in events else -1 for e in ("afterfork2", "join2", "afterjoin1"))
         assert fork >= 0 and fork < join < wait, (k, events)
         assert not any(e.endswith("2") for e in events[join + 1:]), (k, events)
+
+
+@pytest.fixture(scope="module")
+def tuner(tmp_path_factory):
+    exe = linked(TUNER, "tokura_tuner.cu", tmp_path_factory.mktemp("tuner"))
+
+    def run(fail_at, kind):
+        out = subprocess.run([exe, str(fail_at), kind], capture_output=True, text=True, timeout=60, check=True).stdout
+        return [int(v) for v in out.split()]
+    return run
+
+
+@pytest.mark.parametrize("kind", ["plain", "ragged"])
+def test_a_failed_tuning_run_leaves_the_handle_as_it_was(tuner, kind):
+    st, calls, *_ = tuner(-1, kind)
+    assert st == 0 and calls > 10
+    for k in range(calls):
+        st, _, lanes, threads, ragged = tuner(k, kind)
+        assert st == 1 and (lanes, threads, ragged) == (4, 64, 2), k

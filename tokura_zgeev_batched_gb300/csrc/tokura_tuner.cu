@@ -124,8 +124,10 @@ extern "C" TOKURA_API int tokuraAutotune(tokurablas_t* handle, int n_min, int n_
       }
     }
     // The default, which may start in fixed point (an order without a shape of its own takes it).
+    const PlainConfig kept = handle->plain[n];
     handle->plain[n] = PlainConfig{0, 0};
     const PlainConfig chosen = plain_config_for(handle, n, batch_count);
+    handle->plain[n] = kept;
     if (chosen.fixed != 0) {
       cudaError_t err;
       const float ms = time_launches(stream, 2, [&]() {
@@ -133,7 +135,7 @@ extern "C" TOKURA_API int tokuraAutotune(tokurablas_t* handle, int n_min, int n_
                             use_shift_hints(handle, n), &handle->fj);
       }, &err);
       if (err != cudaSuccess) return 1;
-      if (ms < best) continue;
+      if (ms < best) best_cfg = PlainConfig{0, 0};
     }
     handle->plain[n] = best_cfg;
   }
@@ -162,8 +164,10 @@ extern "C" TOKURA_API int tokuraAutotuneRagged(tokurablas_t* handle, int batch_c
   fill_sizes_kernel<<<1, 1, 0, stream>>>(n, off, batch_count, n_min, n_max, 0x5eed1234ULL);
   float best = 1e30f;
   int best_lanes = 0;
+  const int kept = handle->ragged_lanes;
   handle->ragged_lanes = 0;
   const bool fixed = use_fixed_ragged(handle);
+  handle->ragged_lanes = kept;
   for (int lanes : {0, 1, 2, 4, 8}) {  // 0: the default (fixed point, or the lane width chosen per size bin)
     cudaError_t err;
     const float ms = time_launches(stream, 2, [&]() {
