@@ -22,7 +22,7 @@
 namespace tzg {
 
 template <int L>
-inline size_t fixed_hess_shared(int n) {
+constexpr size_t fixed_hess_shared(int n) {
   const int tw = L >= 32 ? 1 : 32 / L;
   return (size_t)tw * fixed_stride<(L > 8 ? 8 : L)>(n * (n | 1) + n) * 16 + (L > 32 ? 32 * 8 : 0);
 }

@@ -6,11 +6,14 @@
 
 namespace tzg {
 
-// Shared memory above the default limit is granted per kernel.
+// Shared memory above the default limit is granted per kernel, for all threads of the process: always as much as the
+// largest launch of any kernel here takes (the reduction's at order 64), so that no call lowers what another has been
+// granted and is about to use.
 template <class Kernel>
 inline cudaError_t allow_shared(Kernel kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  constexpr size_t kDefault = 48 * 1024, kMost = fixed_hess_shared<128>(kMaxN);
+  if (bytes <= kDefault) return cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
 }
 
 // Staging and Hessenberg reduction of the matrices of `work`, of order n at most and `batch` of them at
