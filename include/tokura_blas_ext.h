@@ -343,6 +343,12 @@ TOKURA_API int tokura_zgeev_batched_gpu_noalloc(tokurablas_t* handle, int n, int
  * failure, -2 in the release build (which checks nothing). */
 TOKURA_API int tokuraDebugAttach(void* record);
 
+/* Bounds-checked build only: the matrix accesses of the fixed-point kernels that
+ * have been checked since the library was loaded (their checked pointers count
+ * them; the FP64 kernels' views do not). Synchronizes the device. Returns 0, -1
+ * NULL, 1 on a CUDA failure, -2 in the release build. */
+TOKURA_API int tokuraDebugChecks(unsigned long long* checks);
+
 /* Size in bytes of the static array behind tokura_zgeev_batched_gpu_noalloc (32 MiB). */
 TOKURA_API size_t tokura_zgeev_noalloc_max_bytes(void);
 

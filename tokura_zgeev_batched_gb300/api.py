@@ -70,6 +70,7 @@ _SIGNATURES = {
     "tokuraSetShiftHints": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     "tokuraSetScaledRotations": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     "tokuraDebugAttach": (ctypes.c_int, [ctypes.c_void_p]),
+    "tokuraDebugChecks": (ctypes.c_int, [ctypes.c_void_p]),
     "tokura_zgeev_vectors_batched_gpu": (
         ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 7),
     "tokura_get_zgeev_vectors_workspacesize": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int]),

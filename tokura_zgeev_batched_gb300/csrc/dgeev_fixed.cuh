@@ -24,12 +24,12 @@ inline size_t real_hess_shared(int n) {
   return (size_t)(tw * real_stride<(L > 16 ? 16 : L)>(n * (n | 1) + n) + (L > 32 ? 32 : 0)) * 8;
 }
 // a <- a - 2 u (u . a) on the m entries a[i * es], split among `qs` neighbouring lanes; as reflect_fixed.
-__device__ __forceinline__ void reflect_fixed_real(const Starts& k, long long* a, int es, int m,
+__device__ __forceinline__ void reflect_fixed_real(const Starts& k, Checked<long long> a, int es, int m,
                                                    const int2* __restrict__ u, bool on, int sub, int qs) {
   long long w = 0, hh = 0;
   const int step = qs * es;
   if (on) {
-    const long long* p = a + sub * es;
+    Checked<long long> p = a + sub * es;
     int i = sub;
     for (; i + qs < m; i += 2 * qs, p += 2 * step) {
       const int2 c = u[i], d = u[i + qs];
@@ -55,7 +55,7 @@ __device__ __forceinline__ void reflect_fixed_real(const Starts& k, long long* a
   for (int o = 1; o < qs; o <<= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
   if (!on) return;
   const Limbs t = limbs(-2 * w);
-  long long* p = a + sub * es;
+  Checked<long long> p = a + sub * es;
 #pragma unroll 2
   for (int i = sub; i < m; i += qs, p += step) {
     const int2 c = u[i];
@@ -78,8 +78,9 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) real_hess_kernel(int n, int b
   const int slot = L >= 32 ? 0 : (threadIdx.x & 31) / L;
   const int ld = n | 1, nn = n * n, stride = real_stride<(L > 16 ? 16 : L)>(n * ld + n);
   const long long j = (long long)blockIdx.x * TW + slot;
-  long long* const A = reinterpret_cast<long long*>(fixed_smem) + slot * stride;
-  int2* const U = reinterpret_cast<int2*>(A + n * ld);
+  long long* const a = reinterpret_cast<long long*>(fixed_smem) + slot * stride;
+  const Checked<long long> A = checked(a, 0, n * ld);
+  int2* const U = reinterpret_cast<int2*>(a + n * ld);
   const FixedGroup<L> G(reinterpret_cast<unsigned long long*>(fixed_smem) + TW * stride);
   const Starts k = make_starts(one);
   int st = kStateDone;
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) real_hess_kernel(int n, int b
 
   for (int r = 0; r + 2 < n; ++r) {
     const int m = n - r - 1;
-    long long* const x = A + r * ld + r + 1;
+    const Checked<long long> x = A + r * ld + r + 1;
     unsigned __int128 s = 0;
     bool need = false;
     if (have)
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) real_hess_kernel(int n, int b
         long long v = shift_by(x[i] - kZero, f.q);
         if (i == 0) v += b0 < 0 ? -f.nn : f.nn;
         const Limbs c = scale_coef(limbs(v), f.gv);
-        U[i] = make_int2(c.h, c.l);
+        checked(U, 0, n)[i] = make_int2(c.h, c.l);
       }
     }
     G.sync();
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) real_hess_kernel(int n, int b
     G.sync();
   }
   if (have) {
-    long long* const out = work + j * real_words(n);
+    const Checked<long long> out = checked(work + j * real_words(n), 0, hess_count(n));
     for (int c = 0; c < n; ++c)
       for (int r = G.rank; r <= min(c + 1, n - 1); r += L) out[hess_idx(r, c)] = A[c * ld + r];
   }

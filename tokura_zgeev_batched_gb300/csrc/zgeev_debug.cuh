@@ -6,6 +6,8 @@
 // counter, records the first offending index and redirects the access to
 // element (0, 0) of the same matrix, which is in bounds: nothing traps and
 // nothing waits. The plain kernels also write each matrix's QR sweep count.
+// The fixed-point kernels reach their matrices through Checked<T>, a plain T* in the release build and a pointer
+// with its limits here; those accesses are also counted (tokuraDebugChecks).
 // The release build compiles none of this (the macros expand to nothing).
 //
 // The record is attached with tokuraDebugAttach (the debug library's only
@@ -57,13 +59,43 @@ __device__ __forceinline__ void dbg_index(long long i, long long bound) {
   if (i < 0 || i >= bound) dbg_violation((int)i, -1, (int)(bound > 0x7fffffffLL ? 0x7fffffff : bound));
 }
 
+// A pointer that may be moved anywhere and read or written from `lo` to below `hi`; an access elsewhere is recorded
+// and goes to `lo`.
+static __device__ unsigned long long g_tzg_checks = 0;
+template <class T>
+struct CheckedPtr {
+  T *p, *lo, *hi;
+  __device__ __forceinline__ T& operator*() const {
+    atomicAdd(&g_tzg_checks, 1ull);
+    if (p >= lo && p < hi) return *p;
+    dbg_violation((int)(p - lo), -2, (int)(hi - lo));
+    return *lo;
+  }
+  __device__ __forceinline__ T& operator[](long long i) const { return *(*this + i); }
+  __device__ __forceinline__ T* operator->() const { return &**this; }
+  __device__ __forceinline__ CheckedPtr operator+(long long i) const { return CheckedPtr{p + i, lo, hi}; }
+  __device__ __forceinline__ CheckedPtr& operator+=(long long i) {
+    p += i;
+    return *this;
+  }
+};
+template <class T>
+using Checked = CheckedPtr<T>;
+// The elements p[from] to p[to - 1].
+template <class T>
+__device__ __forceinline__ Checked<T> checked(T* p, long long from, long long to) {
+  return CheckedPtr<T>{p, p + from, p + to};
+}
+
 using DebugAttachFn = cudaError_t (*)(DebugRecord*);
-void debug_register(DebugAttachFn fn);  // tokura_capi.cpp
+using DebugChecksFn = cudaError_t (*)(unsigned long long*);
+void debug_register(DebugAttachFn fn, DebugChecksFn checks);  // zgeev_debug.cu
 
 namespace {
 cudaError_t debug_attach_unit(DebugRecord* rec) { return cudaMemcpyToSymbol(g_tzg_dbg, &rec, sizeof(rec)); }
+cudaError_t debug_checks_unit(unsigned long long* n) { return cudaMemcpyFromSymbol(n, g_tzg_checks, sizeof(*n)); }
 struct DebugUnitRegistration {
-  DebugUnitRegistration() { debug_register(&debug_attach_unit); }
+  DebugUnitRegistration() { debug_register(&debug_attach_unit, &debug_checks_unit); }
 };
 DebugUnitRegistration g_debug_unit_registration;
 }  // namespace
@@ -81,6 +113,13 @@ DebugUnitRegistration g_debug_unit_registration;
   } while (0)
 
 #else
+
+template <class T>
+using Checked = T*;
+template <class T>
+__device__ __forceinline__ T* checked(T* p, long long, long long) {
+  return p;
+}
 
 #define TZG_DBG_TOUCH(view, r, c) ((void)0)
 #define TZG_DBG_INDEX(i, bound) ((void)0)

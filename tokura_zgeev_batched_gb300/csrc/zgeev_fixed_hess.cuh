@@ -137,13 +137,13 @@ struct DotPart {  // conj(u) e, one term: high products and middle products
 };
 
 template <bool kConj>
-__device__ __forceinline__ void reflect_fixed(const Starts& k, cfx* a, int es, int m, const int4* __restrict__ u, Limbs mur,
+__device__ __forceinline__ void reflect_fixed(const Starts& k, Checked<cfx> a, int es, int m, const int4* __restrict__ u, Limbs mur,
                                               Limbs mui, bool on, int sub, int qs) {
   DotPart w = {0, 0, 0, 0};
   long long wx = 0, wy = 0;
   if (on) {
     // Two terms between folds of the middle sums: they stay below 2^63.
-    const cfx* p = a + sub * es;
+    Checked<cfx> p = a + sub * es;
     const int step = qs * es;
     int i = sub;
     for (; i + qs < m; i += 2 * qs, p += 2 * step) {
@@ -193,7 +193,7 @@ __device__ __forceinline__ void reflect_fixed(const Starts& k, cfx* a, int es, i
     hh = mad_wide(mi.h, x.h, hh);
     ty = limbs((hh << 3) + (mid >> 29));
   }
-  cfx* p = a + sub * es;
+  Checked<cfx> p = a + sub * es;
   const int step = qs * es;
 #pragma unroll 2
   for (int i = sub; i < m; i += qs, p += step) {
@@ -284,8 +284,9 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
   const int n = tile.n, ld = n | 1, nn = n * n, stride = fixed_stride<(L > 8 ? 8 : L)>(n * ld + n);
   const long long j = tile.j;
   const bool exists = slot < tile.count;
-  cfx* const A = reinterpret_cast<cfx*>(fixed_smem) + slot * stride;
-  int4* const U = reinterpret_cast<int4*>(A + n * ld);
+  cfx* const a = reinterpret_cast<cfx*>(fixed_smem) + slot * stride;
+  const Checked<cfx> A = checked(a, 0, n * ld);
+  int4* const U = reinterpret_cast<int4*>(a + n * ld);
   const FixedGroup<L> G(reinterpret_cast<unsigned long long*>(fixed_smem + (size_t)TW * stride * 16));
   const Starts k = make_starts(one);
   int st = kStateDone;  // this matrix's state; only exponents go on to the reduction
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
   }
   const bool have = st != kStateDone && st != kStateGeneral;
   if (L > 32 ? !have : !__any_sync(0xffffffffu, have)) continue;  // block- or warp-uniform
-  cfx* const Q = kQ ? q + tile.where + (long long)slot * nn : nullptr;
+  const Checked<cfx> Q = checked(kQ ? q + tile.where + (long long)slot * nn : q, 0, nn);
   if (kQ && have)
     for (int c = 0; c < n; ++c)
       for (int r = G.rank; r < n; r += L) Q[c * n + r] = cfx{r == c ? kFixedOne + kZero : kZero, kZero};
@@ -355,7 +356,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
 
   for (int r = 0; r + 1 < n; ++r) {
     const int m = n - r - 1;
-    cfx* const x = A + r * ld + r + 1;
+    const Checked<cfx> x = A + r * ld + r + 1;
     unsigned __int128 s = 0;
     bool need = false;
     if (have)
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
         v.y = shift_by(v.y - kZero, f.q);
         if (i == 0) v.x += bx < 0 ? -f.nn : f.nn;
         const Limbs ur = scale_coef(limbs(v.x), f.gv), ui = scale_coef(limbs(v.y), f.gv);
-        U[i] = make_int4(ur.h, ur.l, ui.h, ui.l);
+        checked(U, 0, n)[i] = make_int4(ur.h, ur.l, ui.h, ui.l);
       }
     }
     G.sync();
@@ -406,7 +407,8 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
     G.sync();
   }
   if (have) {
-    cfx* const out = hess + tile.where + (long long)slot * (kQ ? nn : hess_stride(n)) + hess_lead(n);
+    const Checked<cfx> out =
+        checked(hess + tile.where + (long long)slot * (kQ ? nn : hess_stride(n)) + hess_lead(n), 0, hess_count(n));
     for (int c = 0; c < n; ++c)
       for (int r = G.rank; r <= min(c + 1, n - 1); r += L) out[hess_idx(r, c)] = A[c * ld + r];
   }

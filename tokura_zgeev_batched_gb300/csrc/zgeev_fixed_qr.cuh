@@ -114,10 +114,11 @@ __device__ __forceinline__ bool nearly_real(cfx a) {
 // ms, 10,000 of n = 32 7.9 -> 9.0.
 template <int L, int T>
 struct QrLane {
-  cfx* H;          // packed matrix
+  Checked<cfx> H;  // packed matrix as read (lanes without work read beyond it)
+  Checked<cfx> W;  // as written
   int4* cur;       // current rotation for columns; then the ring of rows' rotations
   cfx* next;       // entry (k, k) that rotation k is made from (L > 1)
-  long long* sub;  // subdiagonals of the window
+  Checked<long long> sub;  // subdiagonals of the window
   Starts starts;
   int rank, lo, m;
   cfx carry[T];  // this lane's entries in flight, one per index
@@ -170,7 +171,7 @@ struct QrLane {
 #pragma unroll
       for (int t = 0; t < U; ++t) {
         const int i = rank + t * L;
-        if (on && i < m) H[at[t] - (i >= kk ? 1 : k)] = o[t];
+        if (on && i < m) W[at[t] - (i >= kk ? 1 : k)] = o[t];
         if (kk <= m) at[t] += i > kk ? 1 : i == kk ? -1 : k + 1;
         if (L > 1 && i == kk + 1) *next = carry[t];
         ld[t] = H[at[t]];
@@ -264,38 +265,40 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
   }
   const bool have = st != kStateDone && st != kStateGeneral;
   if (!__any_sync(kAll, have)) continue;
-  cfx* H;
+  cfx* h;
   cfx* words = reinterpret_cast<cfx*>(fixed_smem);
   if constexpr (kReal) {
     if (kGlobal) {
-      H = B.scratch + ((long long)blockIdx.x * TW + slot) * (count + 2) + 1;
+      h = B.scratch + ((long long)blockIdx.x * TW + slot) * (count + 2) + 1;
     } else {
-      H = words + 1 + slot * stride;
+      h = words + 1 + slot * stride;
       words += TW * stride;
     }
     if (have) {
       const long long* const src = B.packed + j * real_words(n);
-      for (int e = rank; e < count; e += L) H[e] = cfx{src[e], kZero};
+      for (int e = rank; e < count; e += L) checked(h, 0, count)[e] = cfx{src[e], kZero};
     }
     __syncwarp();
   } else if (kGlobal) {
-    H = hess + tile.where + (long long)min(slot, tile.count - 1) * hess_stride(n) + 1;
+    h = hess + tile.where + (long long)min(slot, tile.count - 1) * hess_stride(n) + 1;
   } else {
-    cfx* const sm = words + 1;
+    const Checked<cfx> sm = checked(words + 1, 0, TW * stride - 1);
     const int all = tile.count * count;
     for (int e = lane; e < all; e += 32) {
       const int t = TW == 1 ? 0 : e / count;
       sm[t * stride + (e - t * count)] = hess[tile.where + t * hess_stride(n) + hess_lead(n) + (e - t * count)];
     }
-    H = sm + slot * stride;
+    h = words + 1 + slot * stride;
     words += TW * stride;
   }
   words += slot * qr_words(n);
+  const Checked<cfx> H = checked(h, -1, count + 1 + qr_slack(n));
   QrLane<L, T> Q;
   Q.H = H;
+  Q.W = checked(h, -1, count + 1);
   Q.cur = reinterpret_cast<int4*>(words);
   Q.next = words + 10;
-  Q.sub = reinterpret_cast<long long*>(words + 11);
+  Q.sub = checked(reinterpret_cast<long long*>(words + 11), 0, n);
   Q.starts = make_starts(one);
   Q.rank = rank;
   if (rank == 0) H[count] = cfx{kZero, kZero};  // row n of the last column
@@ -387,7 +390,7 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
     for (int t = 0; t < T; ++t) {  // H - sigma I
       const int jj = min(lo + rank + t * L, n - 1);
       if (rank + t * L < m) {
-        cfx* const d = H + hess_idx(jj, jj);
+        cfx* const d = &H[hess_idx(jj, jj)];
         d->x -= sigma.x;
         d->y -= sigma.y;
       }
@@ -415,7 +418,7 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
     for (int t = 0; t < T; ++t) {
       const int jj = lo + rank + t * L;
       if (rank + t * L < m) {
-        cfx* const d = H + hess_idx(jj, jj);
+        cfx* const d = &H[hess_idx(jj, jj)];
         d->x += sigma.x;
         d->y += sigma.y;
       }

@@ -28,10 +28,10 @@ inline size_t fixed_schur_shared(int n) {
 
 template <int L, int T>
 struct SchurLane {
-  cfx *H, *Q;      // T (packed), Q (column-major n x n)
+  Checked<cfx> H, W, Q;  // T (packed; as read and as written), Q (column-major n x n)
   int4* cur;       // as QrLane
   cfx* next;
-  long long* sub;
+  Checked<long long> sub;
   Starts starts;
   int rank, n, lo, m;
   cfx carry[2 * T], ld[2 * T];  // T's indices, then Q's rows
@@ -86,7 +86,7 @@ struct SchurLane {
         // Columns right of the window take rotations 0 .. m - 1, indices above it rotations from step 2 on.
         const bool live = rank + t * L < n && (i >= m ? kk < m : i < 0 ? rows : kk <= m + 1);
         if (live) {
-          H[at[t] - (col ? 1 : k)] = o;
+          W[at[t] - (col ? 1 : k)] = o;
           carry[t] = p;
           if (i >= m ? kk + 1 < m : kk <= m) at[t] += i > kk ? 1 : i == kk ? -1 : k + 1;
         }
@@ -157,6 +157,8 @@ struct SchurDone {
   __device__ __forceinline__ long long eig(long long j, int n) const { return offsets != nullptr ? offsets[j] : j * n; }
   __device__ __forceinline__ void entry(const FixedTile& t, int slot, int r, int c, double2 v) const {
     const int p = t.pos + slot, g0 = p / t.width * t.width, tw = min(t.width, t.total - g0);
+    TZG_DBG_INDEX(r, t.n);
+    TZG_DBG_INDEX(c, t.n);
     T[t.origin + (long long)g0 * t.n * t.n + (long long)(c * t.n + r) * tw + (p - g0)] = v;
   }
   __device__ __forceinline__ void deflated(const FixedTile& t, int slot, int i, int k) const {
@@ -192,20 +194,22 @@ __global__ void __launch_bounds__(32) fixed_schur_kernel(Work work, Hint hint, D
     bool have = st != kStateDone && st != kStateGeneral;
     if (!__any_sync(kAll, have)) continue;
     cfx* words = reinterpret_cast<cfx*>(fixed_smem);
-    cfx* const sm = words + 1;
+    const Checked<cfx> sm = checked(words + 1, 0, TW * stride - 1);
     const int all = tile.count * count;
     for (int e = lane; e < all; e += 32) {
       const int t = TW == 1 ? 0 : e / count;
       sm[t * stride + (e - t * count)] = hess[tile.where + (long long)t * nn + hess_lead(n) + (e - t * count)];
     }
-    cfx* const H = sm + slot * stride;
+    cfx* const h = words + 1 + slot * stride;
+    const Checked<cfx> H = checked(h, -1, count + 1 + qr_slack(n));
     words += TW * stride + slot * schur_words(n);
     SchurLane<L, T> S;
     S.H = H;
-    S.Q = q + mine;
+    S.W = checked(h, -1, count + 1);
+    S.Q = checked(q + mine, 0, nn);
     S.cur = reinterpret_cast<int4*>(words);
     S.next = words + 10;
-    S.sub = reinterpret_cast<long long*>(words + 11);
+    S.sub = checked(reinterpret_cast<long long*>(words + 11), 0, n);
     cfx* const list = words + qr_words(n);
     S.starts = make_starts(one);
     S.rank = rank;
@@ -344,7 +348,7 @@ __global__ void __launch_bounds__(32) fixed_schur_kernel(Work work, Hint hint, D
       for (int t = 0; t < T; ++t) {  // H - sigma I on the window
         const int i = rank + t * L - lo;
         if (i >= 0 && i < m) {
-          cfx* const d = H + hess_idx(lo + i, lo + i);
+          cfx* const d = &H[hess_idx(lo + i, lo + i)];
           d->x -= sigma.x;
           d->y -= sigma.y;
           S.sub[i] = H[hess_idx(lo + i + 1, lo + i)].x;
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(32) fixed_schur_kernel(Work work, Hint hint, D
       for (int t = 0; t < T; ++t) {
         const int i = rank + t * L - lo;
         if (i >= 0 && i < m) {
-          cfx* const d = H + hess_idx(lo + i, lo + i);
+          cfx* const d = &H[hess_idx(lo + i, lo + i)];
           d->x += sigma.x;
           d->y += sigma.y;
         }
