@@ -207,3 +207,33 @@ def test_badly_balanced_matrices_are_left_to_fp64(cuda, n):
     assert h.set_real_config(n, 8 if n >= 16 else 4, 32) == 0
     for got, ref in zip(api.dgeev_batched(R), api.dgeev_batched(R, handle=h)):
         assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("n", [33, 47, 64])
+def test_real_matrices_with_repeated_eigenvalues(cuda, n):
+    """Given up as soon as two eigenvalues have one place: the FP64 kernel's results, the others as without them."""
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    rng = np.random.default_rng(6800 + n)
+    A = rng.standard_normal((40, n, n))
+    Q = np.linalg.qr(A)[0]
+    A[3] = Q[3][:, : n // 2] @ Q[3][:, : n // 2].T  # a projection
+    A[8] = np.eye(n)[rng.permutation(n)]
+    A[9] = np.kron(np.eye(n // 2 + 1), [[0.5, 2.0], [-1.0, 0.25]])[:n, :n]  # one pair many times
+    A[11] = 0.0
+    A[11, np.arange(1, n), np.arange(n - 1)] = 1.0  # a cycle: no two alike
+    A[11, 0, n - 1] = 1.0
+    M = torch.from_numpy(A).cuda()
+    h = api.Handle()
+    assert h.set_real_config(n, 8, 32) == 0  # what so small a batch uses
+    got, ref = api.dgeev_batched(M), api.dgeev_batched(M, handle=h)
+    for g, r in zip(got, ref):
+        assert torch.equal(g[[3, 8, 9]], r[[3, 8, 9]])
+    others = [k for k in range(40) if k not in (3, 8, 9)]
+    for g, r in zip(got, api.dgeev_batched(M[others].contiguous())):
+        assert torch.equal(g[others], r)
+    wr, wi, f = got
+    assert not f.any()
+    err = lo.matched_abs_errors(torch.complex(wr, wi)[11:12].cpu().numpy(), np.exp(2j * np.pi * np.arange(n) / n)[None])
+    assert err.max() <= lo.TOL_REL_FRO * np.sqrt(n)

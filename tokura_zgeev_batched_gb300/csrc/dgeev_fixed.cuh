@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) real_hess_kernel(int n, int b
       if (G.rank == 0) flag[j] = (char)(emax != 0 ? kNonFinite : kConverged);
     } else {
       G.sync();
+      st = kStateGeneral;
       float s2 = 0.0f;
       const bool left = left_to_fp64(G, n, emax, [&](int r, int c) {
         const long long z = A[c * ld + r];
@@ -111,18 +112,19 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) real_hess_kernel(int n, int b
         return size_of(z);
       }, [&](int r, int c) { return size_of(A[c * ld + r]); }, reinterpret_cast<int*>(U));
       G.sync();
-      const int p = exponent_of(kFixedNormMax / mulf(sqrtf(G.sumf(s2)), 1.0001f));
-      unsigned long long lower = 0, upper = 0;  // as for complex matrices
-      for (int c = G.rank; c < n; c += L)
-        for (int r = 0; r < n; ++r) {
-          const long long w = to_fixed(A[c * ld + r], emax, p);
-          A[c * ld + r] = w;
-          const unsigned long long v = mag64(w - kZero);
-          if (r > c) lower |= v;
-          if (r < c) upper |= v;
-        }
-      const bool full = G.ior((lower != 0 ? 1u : 0u) | (upper != 0 ? 2u : 0u)) == 3;
-      st = left || !full ? kStateGeneral : emax - 1023 - p;
+      if (!left) {
+        const int p = exponent_of(kFixedNormMax / mulf(sqrtf(G.sumf(s2)), 1.0001f));
+        unsigned long long lower = 0, upper = 0;  // as for complex matrices
+        for (int c = G.rank; c < n; c += L)
+          for (int r = 0; r < n; ++r) {
+            const long long w = to_fixed(A[c * ld + r], emax, p);
+            A[c * ld + r] = w;
+            const unsigned long long v = mag64(w - kZero);
+            if (r > c) lower |= v;
+            if (r < c) upper |= v;
+          }
+        if (G.ior((lower != 0 ? 1u : 0u) | (upper != 0 ? 2u : 0u)) == 3) st = emax - 1023 - p;
+      }
     }
     if (G.rank == 0) {
       work[(j + 1) * real_words(n) - 1] = st == kStateGeneral ? kStateDone : st;

@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
         if (G.rank == 0) flag[j] = (char)(emax != 0 ? kNonFinite : kConverged);
       } else {
         G.sync();
+        st = kStateGeneral;
         float s2 = 0.0f;
         const auto size = [&](int r, int c) {
           const cfx z = A[c * ld + r];
@@ -326,22 +327,23 @@ __global__ void __launch_bounds__(L > 32 ? L : 32) fixed_hess_kernel(Work work, 
           return max(size_of(z.x), size_of(z.y));
         }, size, reinterpret_cast<int*>(U));
         G.sync();
-        const float top = kFixedNormMax / mulf(sqrtf(G.sumf(s2)), 1.0001f);
-        const int p = exponent_of(top);
-        // Fixed point. Triangular matrices are left to the FP64 kernels too (an upper triangular one's diagonal is
-        // exact there).
-        unsigned long long lower = 0, upper = 0;
-        for (int c = G.rank; c < n; c += L)
-          for (int r = 0; r < n; ++r) {
-            const cfx z = A[c * ld + r];
-            const cfx w = {to_fixed(z.x, emax, p), to_fixed(z.y, emax, p)};
-            A[c * ld + r] = w;
-            const unsigned long long v = mag64(w.x - kZero) | mag64(w.y - kZero);
-            if (r > c) lower |= v;
-            if (r < c) upper |= v;
-          }
-        const bool full = G.ior((lower != 0 ? 1u : 0u) | (upper != 0 ? 2u : 0u)) == 3;
-        st = left || !full ? kStateGeneral : emax - 1023 - p;
+        if (!left) {
+          const float top = kFixedNormMax / mulf(sqrtf(G.sumf(s2)), 1.0001f);
+          const int p = exponent_of(top);
+          // Fixed point. Triangular matrices are left to the FP64 kernels too (an upper triangular one's diagonal is
+          // exact there).
+          unsigned long long lower = 0, upper = 0;
+          for (int c = G.rank; c < n; c += L)
+            for (int r = 0; r < n; ++r) {
+              const cfx z = A[c * ld + r];
+              const cfx w = {to_fixed(z.x, emax, p), to_fixed(z.y, emax, p)};
+              A[c * ld + r] = w;
+              const unsigned long long v = mag64(w.x - kZero) | mag64(w.y - kZero);
+              if (r > c) lower |= v;
+              if (r < c) upper |= v;
+            }
+          if (G.ior((lower != 0 ? 1u : 0u) | (upper != 0 ? 2u : 0u)) == 3) st = emax - 1023 - p;
+        }
       }
     }
     if (G.rank == 0) *(kQ ? schur_state(hess + tile.where + (long long)slot * nn, n) : state + j) = st;

@@ -102,6 +102,11 @@ __device__ __forceinline__ bool conjugates(cfx a, cfx b) {
   return mag64(a.x - b.x) <= (unsigned long long)kConjugateUnits &&
          mag64(a.y - kZero + (b.y - kZero)) <= (unsigned long long)kConjugateUnits;
 }
+// Two eigenvalues so close that their conjugates, if found where they must be, will have two partners each.
+__device__ __forceinline__ bool together(cfx a, cfx b) {
+  return mag64(a.x - b.x) <= (unsigned long long)(kConjugateUnits / 4) &&
+         mag64(a.y - b.y) <= (unsigned long long)(kConjugateUnits / 4);
+}
 __device__ __forceinline__ bool nearly_real(cfx a) {
   return mag64(a.y - kZero) <= (unsigned long long)(kConjugateUnits / 2);
 }
@@ -336,6 +341,7 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
         small |= (unsigned long long)vote << (t * L);
       }
     }
+    const int last = hi;
     while (hi >= 0) {
       const unsigned long long below = small & ((2ull << hi) - 1ull);
       lo = below ? 63 - clz64(below) : 0;
@@ -349,6 +355,30 @@ __global__ void __launch_bounds__(32) fixed_qr_kernel(Work work, Batch B, cfx* _
       --hi;
       its = 0;
       kdefl = 0;
+    }
+    if constexpr (kReal && L * T > 32) {
+      // Two eigenvalues at one place (or a real one with a partner) will not pair: no need to see the others. From order
+      // 33 on (16,384 of order 64: projections 63.5 -> 54.4 ms, permutations 134 -> 112, Gaussian ones 61.2 -> 60.4); below,
+      // Gaussian ones pay for it (10,000 of 32 5.77 -> 5.84, 65,536 of 16 5.39 -> 5.87, 300,000 of 4 0.98 -> 1.10).
+      if (__any_sync(kAll, hi < last)) {
+        bool clash = false;
+        for (int p = last; p > hi; --p) {
+          const cfx d = H[hess_idx(p, p)];
+          const bool real = nearly_real(d);
+#pragma unroll
+          for (int t = 0; t < T; ++t) {
+            const int i = rank + t * L;
+            if (i <= p || i >= n) continue;
+            const cfx e = H[hess_idx(i, i)];
+            clash |= together(d, e) || (real && conjugates(d, e));
+          }
+        }
+        const unsigned vote = __ballot_sync(kAll, clash) >> base;
+        if ((L == 32 ? vote : vote & ((1u << (L & 31)) - 1u)) != 0) {
+          status = kNotConverged;
+          hi = -1;
+        }
+      }
     }
     if (hi >= 0 && its > itmax) {
       status = kNotConverged;
