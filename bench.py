@@ -13,7 +13,8 @@ pinned host memory and the eigenvalues/flags copied back inside every step.
 per matrix over all host cores, stream_test_with_MKL/get_eig_MKL.c:27-47) on
 a bounded sample of the same workload. Under torchrun every rank processes its
 own batch (weak scaling, no collective on the data path); rank 0 prints the
-JSON line with the max time over ranks.
+JSON line with the max time over ranks, and the whole record, every
+configuration with its details, on stderr before it.
 """
 from __future__ import annotations
 
@@ -251,8 +252,46 @@ def run_reference(args):
 
 # ----------------------------------------------------------------------------- our arm
 
+# What the line on stdout keeps of the timed workload's own sections; everything else that was measured
+# goes to stderr, whole.
+LINE_KEYS = {
+    "config": ("workload", "n", "global_batch", "l2"),
+    "roofline": ("achieved", "peak", "unit", "frac", "int_mad"),
+    "cpu_baseline": ("value", "unit", "cores", "kind", "error"),
+    "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "error"),
+    "clocks": ("sm_mhz", "sm_max_mhz", "reasons"),
+    "parity": ("checked", "flag_mismatch", "max_rel_err_fro", "error"),
+}
+LINE_BYTES = 1400
+
+
+def short_line(out: dict) -> str:
+    """The benchmark's line: the timed workload with its sections cut to LINE_KEYS, then of each
+    further configuration its own numbers, as many configurations as LINE_BYTES has room for (a
+    line of some 20 KB does not survive a log that keeps the last one or two)."""
+    def rounded(v):
+        if isinstance(v, float):
+            return float(f"{v:.6g}")
+        if isinstance(v, dict):
+            return {k: rounded(x) for k, x in v.items() if not isinstance(x, str)}
+        return v
+
+    line, rest = {}, {}
+    for key, v in out.items():
+        if not isinstance(v, dict):
+            line[key] = v
+        elif key in LINE_KEYS:
+            line[key] = {k: rounded(v[k]) for k in LINE_KEYS[key] if k in v}
+        else:
+            rest[key] = {k: rounded(x) for k, x in v.items() if isinstance(x, (int, float)) or k == "error"}
+    for key, v in rest.items():
+        if v and len(json.dumps({**line, key: v})) <= LINE_BYTES:
+            line[key] = v
+    return json.dumps(line)
+
+
 def phase(name: str) -> None:
-    """Progress marker on stderr (the JSON line is the only stdout output)."""
+    """Progress marker on stderr (the short JSON line is the only stdout output)."""
     print(f"[bench {time.strftime('%H:%M:%S')}] {name}", file=sys.stderr, flush=True)
 
 
@@ -1203,7 +1242,8 @@ def run_ours(args):
             "config5_ragged_gd_graph": config5, "real_dgeev_n64": real, "eigenvectors_n64": vectors,
             "reference_gpu": reference_gpu,
         }
-        print(json.dumps(out), flush=True)
+        print(json.dumps(out), file=sys.stderr, flush=True)
+        print(short_line(out), flush=True)
     if dist is not None:
         dist.destroy_process_group()
 
