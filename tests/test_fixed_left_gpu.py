@@ -237,3 +237,26 @@ def test_real_matrices_with_repeated_eigenvalues(cuda, n):
     assert not f.any()
     err = lo.matched_abs_errors(torch.complex(wr, wi)[11:12].cpu().numpy(), np.exp(2j * np.pi * np.arange(n) / n)[None])
     assert err.max() <= lo.TOL_REL_FRO * np.sqrt(n)
+
+
+@pytest.mark.parametrize("n,batch", [(5, 40001), (9, 40001), (16, 20001), (20, 9801), (33, 9801), (64, 9801)])
+def test_few_left_matrices_in_a_large_batch(cuda, n, batch):
+    """Alone or one in eight of a warp's tile: the bits of a small FP64 batch; more of them: parity, as the batch's."""
+    import torch
+    from tokura_zgeev_batched_gb300 import api
+
+    M = wl.torch_gaussian(batch, n, seed=6900 + n)
+    d = torch.from_numpy(2.0 ** np.linspace(0, -30, n)).cuda()
+    few, many = [3, 9000, batch - 1], list(range(640, 672))
+    plain = api.zgeev_batched(M)[0]
+    for j in few + many:
+        M[j] *= d[:, None] * d
+    w, f = api.zgeev_batched(M)
+    assert not f.any()
+    alone = api.zgeev_batched(M[few].contiguous(), handle=fp64_handle())[0]
+    assert np.array_equal(bits(w[few]), bits(alone))
+    others = torch.ones(batch, dtype=torch.bool, device="cuda")
+    others[few + many] = False
+    assert torch.equal(torch.view_as_real(w[others]), torch.view_as_real(plain[others]))
+    err = lo.matched_abs_errors(w[many].cpu().numpy(), lo.zgeev(M[many].cpu().numpy())[0])
+    assert (err.max(1) <= lo.TOL_REL_FRO * torch.linalg.norm(M[many], dim=(1, 2)).cpu().numpy()).all()

@@ -136,8 +136,7 @@ inline PlainConfig plain_config_for(const tokurablas_t* h, int n, int batch) {
     else if ((long long)batch * 4 >= want_lanes)
       c.lanes = 4;
     else {
-      int cap = 32;
-      while (cap > 4 && cap > n / 2) cap >>= 1;
+      const int cap = few_lanes(n);
       c.lanes = 4;
       while (c.lanes < cap && (long long)batch * c.lanes < want_lanes) c.lanes <<= 1;
     }

@@ -22,6 +22,14 @@ struct PlainConfig {
 // Iteration cap per eigenvalue: LAPACK's rule 30*max(10, n) unless overridden.
 __host__ __device__ inline int default_itmax(int n) { return 30 * (n > 10 ? n : 10); }
 
+// Lanes per matrix of the plain kernel where a few matrices have the GPU to themselves: two elements of a row or
+// column for each lane, 4 to 32.
+inline int few_lanes(int n) {
+  int lanes = 32;
+  while (lanes > 4 && lanes > n / 2) lanes >>= 1;
+  return lanes;
+}
+
 // Launches the fused stage + Hessenberg + QR kernel on `stream`.
 // `work` must hold 16*n*n*batch bytes (tile-interleaved copy of A).
 // A second stream and two events for running the FP32 estimator beside the

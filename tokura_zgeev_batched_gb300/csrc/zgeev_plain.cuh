@@ -83,6 +83,13 @@ struct Complex64Batch {
   __device__ __forceinline__ float2* out(long long j, int) const { return W + j * n; }
 };
 
+// Which of the matrices that fixed point left a launch takes, by how many of `tile` neighbours were left: few (one in
+// eight at most, or one alone) or more. tile 0: all.
+struct LeftRule {
+  int tile = 0;
+  bool few = false;
+};
+
 // `scaled` (nonzero, n >= kScaledMinN) selects the QR with scaled rotations
 // (zgeev_scaled_qr.cuh) for the QR part; the prepare part does not depend on it.
 // Warp w solves matrices w*32/L .. w*32/L + 32/L - 1 with L lanes each. The
@@ -93,7 +100,7 @@ template <int L, bool kBalance, int kPhase, class Batch>
 __global__ void __launch_bounds__(256) zgeev_plain_kernel(int n, int batch, Batch B, double2* __restrict__ work,
                                                            char* __restrict__ flag, int itmax, int balance,
                                                            const float2* __restrict__ est, int* __restrict__ state,
-                                                           int scaled, int stage_tw) {
+                                                           int scaled, int stage_tw, LeftRule rule) {
   constexpr int TW = 32 / L;  // matrices per warp (1 at 32 lanes)
   const int lane = threadIdx.x & 31;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -104,7 +111,15 @@ __global__ void __launch_bounds__(256) zgeev_plain_kernel(int n, int batch, Batc
   const long long t0 = j / stage_tw * stage_tw;  // first matrix of j's staging tile
   MatView M{work + t0 * nn + (j - t0), n, (int)min((long long)stage_tw, (long long)batch - t0)};
   // After the fixed-point kernels: only the matrices that they left (group-uniform).
-  if (kPhase == kPhaseAll && state != nullptr && state[j] != kStateGeneral) return;
+  if (kPhase == kPhaseAll && state != nullptr) {
+    if (state[j] != kStateGeneral) return;
+    if (rule.tile != 0) {
+      const long long first = j / rule.tile * rule.tile, end = min(first + rule.tile, (long long)batch);
+      int left = 0;
+      for (long long i = first; i < end; ++i) left += state[i] == kStateGeneral ? 1 : 0;
+      if ((left <= rule.tile / 8 || left == 1) != rule.few) return;
+    }
+  }
 
   if (kPhase != kPhaseQR && !B.valid(j)) {  // NULL matrix pointer: NaN eigenvalues, flag 3 (group-uniform)
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
@@ -154,14 +169,15 @@ __global__ void __launch_bounds__(256) zgeev_plain_kernel(int n, int batch, Batc
 template <int L, bool kBalance, int kPhase, class Batch>
 inline cudaError_t launch_plain_l(unsigned blocks, int threads, cudaStream_t stream, int n, int batch,
                                   const Batch& B, double2* work, char* flag, int itmax, int balance,
-                                  const float2* est, int* state, int carveout, int scaled, int stage_tw) {
+                                  const float2* est, int* state, int carveout, int scaled, int stage_tw,
+                                  LeftRule rule) {
   if (kPhase != kPhaseAll) {  // shared memory for estimators running beside (this or another call's)
     const cudaError_t err = cudaFuncSetAttribute(zgeev_plain_kernel<L, kBalance, kPhase, Batch>,
                                                  cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
     if (err != cudaSuccess) return err;
   }
   zgeev_plain_kernel<L, kBalance, kPhase, Batch>
-      <<<blocks, threads, 0, stream>>>(n, batch, B, work, flag, itmax, balance, est, state, scaled, stage_tw);
+      <<<blocks, threads, 0, stream>>>(n, batch, B, work, flag, itmax, balance, est, state, scaled, stage_tw, rule);
   return cudaGetLastError();
 }
 
@@ -170,41 +186,42 @@ inline cudaError_t launch_plain_l(unsigned blocks, int threads, cudaStream_t str
 template <int kPhase, class Batch>
 inline cudaError_t launch_plain_phase(int L, bool bal, unsigned blocks, int threads, cudaStream_t stream, int n,
                                       int batch, const Batch& B, double2* work, char* flag, int itmax, int balance,
-                                      const float2* est, int* state, int carveout, int scaled, int stage_tw) {
+                                      const float2* est, int* state, int carveout, int scaled, int stage_tw,
+                                      LeftRule rule = LeftRule()) {
   constexpr bool kB = kPhase != kPhaseQR;  // balanced instantiation exists
   const bool b = bal && kB;
   const int bv = b ? balance : 0;
   switch (L) {
     case 1:
       return b ? launch_plain_l<1, kB, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, bv, est, state,
-                                                        carveout, scaled, stage_tw)
+                                                        carveout, scaled, stage_tw, rule)
                : launch_plain_l<1, false, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, 0, est, state,
-                                                           carveout, scaled, stage_tw);
+                                                           carveout, scaled, stage_tw, rule);
     case 2:
       return b ? launch_plain_l<2, kB, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, bv, est, state,
-                                                        carveout, scaled, stage_tw)
+                                                        carveout, scaled, stage_tw, rule)
                : launch_plain_l<2, false, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, 0, est, state,
-                                                           carveout, scaled, stage_tw);
+                                                           carveout, scaled, stage_tw, rule);
     case 4:
       return b ? launch_plain_l<4, kB, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, bv, est, state,
-                                                        carveout, scaled, stage_tw)
+                                                        carveout, scaled, stage_tw, rule)
                : launch_plain_l<4, false, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, 0, est, state,
-                                                           carveout, scaled, stage_tw);
+                                                           carveout, scaled, stage_tw, rule);
     case 8:
       return b ? launch_plain_l<8, kB, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, bv, est, state,
-                                                        carveout, scaled, stage_tw)
+                                                        carveout, scaled, stage_tw, rule)
                : launch_plain_l<8, false, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, 0, est, state,
-                                                           carveout, scaled, stage_tw);
+                                                           carveout, scaled, stage_tw, rule);
     case 16:
       return b ? launch_plain_l<16, kB, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, bv, est, state,
-                                                        carveout, scaled, stage_tw)
+                                                        carveout, scaled, stage_tw, rule)
                : launch_plain_l<16, false, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, 0, est, state,
-                                                           carveout, scaled, stage_tw);
+                                                           carveout, scaled, stage_tw, rule);
     case 32:
       return b ? launch_plain_l<32, kB, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, bv, est, state,
-                                                        carveout, scaled, stage_tw)
+                                                        carveout, scaled, stage_tw, rule)
                : launch_plain_l<32, false, kPhase>(blocks, threads, stream, n, batch, B, work, flag, itmax, 0, est, state,
-                                                           carveout, scaled, stage_tw);
+                                                           carveout, scaled, stage_tw, rule);
     default:
       return cudaErrorInvalidValue;
   }
@@ -238,8 +255,23 @@ cudaError_t launch_batch(const PlainConfig& cfg, int n, int batch, const Batch& 
     const cudaError_t e = launch_fixed(n, batch, cfg.fixed, B, reinterpret_cast<cfx*>(work), flag, itmax, left,
                                        stream);
     if (e != cudaSuccess) return e;
+    // A few left matrices in a large batch would each be a chain on the batch's few lanes: they get a launch with the
+    // lanes of a small batch, and the narrow one takes what has more left neighbours. One graded matrix in a batch:
+    // 65,536 of order 64 453.6 -> 354.3 ms (346 without it), 10,000 of 32 13.2 -> 10.5 (7.9), 65,536 of 16 9.0 -> 7.4 (6.6).
+    // Up to order 4 the chain is short and the launch shows (1,048,576 of 4: 0.06 ms with one launch).
+    const int wide = few_lanes(n);
+    LeftRule rule;
+    if (n > 4 && wide > L) {
+      const long long warps = ((long long)batch * wide + 31) / 32;  // four to a block
+      rule = LeftRule{tw, true};
+      const cudaError_t w = launch_plain_phase<kPhaseAll>(wide, false, (unsigned)((warps + 3) / 4), 128, stream, n, batch,
+                                                          B, work, flag, itmax, 0, nullptr, left, kDef, 0, 32 / wide,
+                                                          rule);
+      if (w != cudaSuccess) return w;
+      rule.few = false;
+    }
     return launch_plain_phase<kPhaseAll>(L, false, (unsigned)blocks, threads, stream, n, batch, B, work, flag, itmax, 0,
-                                         nullptr, left, kDef, scaled, tw);
+                                         nullptr, left, kDef, scaled, tw, rule);
   }
   if (!hints)
     return launch_plain_phase<kPhaseAll>(L, bal, (unsigned)blocks, threads, stream, n, batch, B, work, flag, itmax,
