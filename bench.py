@@ -38,15 +38,18 @@ SWEEP_NS = (4, 8, 16, 32, 48)  # the size sweep's other orders (n = 64 is the ti
 
 
 # A plain call with the library's choices is three kernels: Hessenberg reduction and QR in 64-bit
-# fixed point, and the FP64 kernel for the matrices that these leave. With a launch shape set
+# fixed point, and the FP64 kernel for the matrices that these leave, twice if the batch's lanes per
+# matrix are fewer than a small batch would get. With a launch shape set
 # (--lanes) it is the FP64 path: an FP32 estimator, the Hessenberg phase and the QR phase from n = 12 on.
 SHIFT_HINT_MIN_N = 12
 
 
-def launches_per_call(n: int, lanes: int) -> int:
+def launches_per_call(n: int, lanes: int, chosen: int) -> int:
+    """``lanes``: set on the handle (0: none); ``chosen``: by the library for this batch."""
     if lanes:
         return 3 if n >= SHIFT_HINT_MIN_N else 1
-    return 3 if n > 1 else 1
+    few = max([w for w in (4, 8, 16, 32) if w <= n // 2] + [4])
+    return 1 if n < 2 else 4 if n > 4 and few > chosen else 3
 
 
 def set_workload(n: int, batch: int = 0) -> None:
@@ -1237,7 +1240,7 @@ def run_ours(args):
                                      "64-bit fixed point on the integer multiplier, FP64 for what that leaves; "
                                      "errors against extended precision below the FP64 kernels'"},
             "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clocks,
-            "gpu_launches": args.steps * launches_per_call(N, args.lanes), "flagged": flagged, "parity": parity, "sweep": sweep,
+            "gpu_launches": args.steps * launches_per_call(N, args.lanes, h.plain_config(N, BATCH)[0]), "flagged": flagged, "parity": parity, "sweep": sweep,
             "config1_n32_10000": config1, "ragged": ragged, "config4_backward": config4,
             "config5_ragged_gd_graph": config5, "real_dgeev_n64": real, "eigenvectors_n64": vectors,
             "reference_gpu": reference_gpu,

@@ -101,8 +101,8 @@ TOKURA_API int tokuraSetPlainQrLanes(tokurablas_t* handle, int n, int lanes_per_
  * host-buffer, workspace-free and ragged eigenvalue calls, the eigenvector
  * call and the ragged gradients start in 64-bit fixed point
  * (csrc/zgeev_fixed.cuh: the matrix as 64-bit integers with one exponent,
- * errors below the FP64 kernels' in norm; graded and triangular matrices are
- * left to those) unless the handle has a launch shape, rotation kind, shift
+ * errors below the FP64 kernels' in norm; graded, badly balanced and
+ * triangular matrices are left to those) unless the handle has a launch shape, rotation kind, shift
  * strategy or balancing set. The uniform gradient, whose results depend on the
  * last bits of the forward where a spectrum is ill-conditioned, takes this
  * call's eigenvalues in the torch binding. Arguments and return codes as
@@ -293,9 +293,11 @@ TOKURA_API int tokura_cgeev_batched_gpu(tokurablas_t* handle, int n, int batch_c
  * conjugates; real eigenvalues have wi exactly 0. Orders of 3 and more are
  * computed in 64-bit fixed point (a real Householder reduction, the complex QR,
  * eigenvalues paired at the end); smaller orders, matrices that this leaves
- * (graded, triangular, conjugates not clear) and calls on a handle with a launch
- * shape or balancing by a real reduction and the Francis double-shift QR in
- * FP64. flag[j] as for
+ * (graded, badly balanced, triangular, repeated eigenvalues or conjugates not
+ * clear) and calls on a handle with a launch shape or balancing by a real
+ * reduction and the Francis double-shift QR in FP64. Batches whose matrices all
+ * have repeated eigenvalues (projections, permutations) are faster with a launch
+ * shape: the fixed-point iteration is given up on them. flag[j] as for
  * tokura_zgeev_batched_gpu (balancing per tokuraSetBalancing, sweep cap per
  * tokuraSetSweepCap). work: tokura_get_dgeev_workspacesize(n, batch_count)
  * bytes. A is read only. Returns 0; -1 NULL handle, -2 bad n, -3 A NULL,

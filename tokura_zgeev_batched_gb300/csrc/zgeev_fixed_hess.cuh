@@ -9,8 +9,8 @@
 // left over: a dot product with u (integer sums; the halves' cross terms are
 // folded in every two terms, so they cannot overflow) and an update.
 //
-// What bounds it: the 32x32-bit multiplier, 12 instructions of four clocks a term, 64 % busy at n = 64 (65,536
-// matrices 87 ms; the FP64 reduction 197); its shared-memory reads and writes take 75 % of that time. A
+// What bounds it: the 32x32-bit multiplier, 12 instructions of four clocks a term, about 60 % busy at n = 64 by
+// instruction counts and times (65,536 matrices 87 ms; the FP64 reduction 197); its shared-memory reads and writes take 75 % of that time. A
 // 64 x 64 matrix is 67 KB, so an SM holds three, and L = 128 lanes each give it 12 warps. Longer unrolls (four
 // terms) changed nothing.
 #pragma once

@@ -112,9 +112,9 @@ __device__ __forceinline__ bool nearly_real(cfx a) {
 }
 
 // Everything a lane keeps during a sweep. What bounds it: the 32x32-bit multiplier, one warp
-// instruction in four clocks of a sub-partition (a rotation is 36 of them, its coefficients 22), 60 % busy
-// at n = 16 (65,536 matrices, 9 warps per SM) and 50 % at n = 64 in shared memory (5.4 warps per SM); the rest is
-// the chain of a step with few warps to hide it. Making rotation k + 1 beside step
+// instruction in four clocks of a sub-partition (a rotation is 36 of them, its coefficients 22), about 60 % busy
+// by instruction counts and times (16,384 matrices of n = 64 in the workspace, 24 warps per SM; the counters give the
+// pipe's instructions, 41 % of its peak, not how long a product holds it); the rest is the chain of a step. Making rotation k + 1 beside step
 // k's work (18 more multiplications and two more loads in every lane) was slower: 16,384 matrices of n = 64 87.2 -> 116.5
 // ms, 10,000 of n = 32 7.9 -> 9.0.
 template <int L, int T>
@@ -192,7 +192,8 @@ struct QrLane {
         sweep<1>(last);
       else
         sweep<2>(last);
-    } else if constexpr (T == 4) {
+    } else {
+      static_assert(T == 4, "indices per lane");
       if (used <= 1)
         sweep<1>(last);
       else if (used == 2)
@@ -201,13 +202,6 @@ struct QrLane {
         sweep<3>(last);
       else
         sweep<4>(last);
-    } else {
-      if (used <= 2)
-        sweep<2>(last);
-      else if (used <= 4)
-        sweep<4>(last);
-      else
-        sweep<T>(last);
     }
   }
 };

@@ -3,10 +3,10 @@
 //   caller's stream: [planning] --fork-- [orders 49..64, 33..48] --join-- [FP64: what was left]
 //   second stream:                 \---- [orders 25..32 .. 2..4] --/
 // The classes above n = 32 keep their matrices in the workspace and the others in shared memory, so the two
-// streams' kernels fit on an SM together, and one's last, half-empty wave is filled by the other. From 100 matrices per
-// SM on the waves are many and what the two evict from each other's caches costs more: all on the caller's
-// stream. Orders in U{1..64}, two streams and one: 1,000 matrices 9.6 and 12.0 ms, 4,000 13.0 and 14.2, 9,000 22.7 and 20.3,
-// 13,000 24.0 and 26.2, 20,000 45.4 and 37.2, 60,000 117 and 100, 200,000 397 and 319.
+// streams' kernels fit on an SM together, and one's last, half-empty wave is filled by the other. In large batches the waves are many and what the two evict from each other's caches costs more: all on the caller's
+// stream. The limit, 100 matrices per SM of any order (15,200 on 152 SMs), lies between measurements that do not agree on one: orders
+// in U{1..64}, two streams and one, 1,000 matrices 9.6 and 12.0 ms, 4,000 13.0 and 14.2, 9,000 22.7 and 20.3, 13,000 24.0
+// and 26.2, 20,000 45.4 and 37.2, 60,000 117 and 100, 200,000 397 and 319; other ranges of orders were not measured.
 #include "zgeev_ragged_work.cuh"
 
 namespace tzg {
