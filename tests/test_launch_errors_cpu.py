@@ -1,6 +1,7 @@
-"""Launch errors on the host, without a GPU: the library's own object files against a stand-in for the CUDA runtime that
+"""The host side without a GPU: the library's own object files against a stand-in for the CUDA runtime that
 counts launches, fails the one it is told to, and writes down what reaches which stream. Work that was forked to the
-handle's second stream is joined again whatever fails after it."""
+handle's second stream is joined again whatever fails after it; a failed tuning run changes nothing; only chunks whose
+matrices share the L2 cache are solved in turn."""
 import os
 import subprocess
 import sys
@@ -130,6 +131,42 @@ int main(int argc, char** argv) {
 }
 """
 
+HOST = RUNTIME + r"""
+#include "tokura_handle.h"
+#include "tokura_blas_ext.h"
+static long waits = 0, solves = 0;
+namespace tzg {
+cudaError_t launch_plain(const PlainConfig&, int, int, const double2*, double2*, double2*, char*, int, cudaStream_t, int,
+                         bool, const ForkJoin*) {
+  ++solves;
+  return cudaSuccess;
+}
+}
+extern "C" {
+static size_t next = 1000;
+cudaError_t cudaMalloc(void** p, size_t) { *p = (void*)4096; return cudaSuccess; }
+cudaError_t cudaFree(void*) { return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)next++; return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)next++; return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void*, const void*, size_t, cudaMemcpyKind, cudaStream_t) { return cudaSuccess; }
+}
+int main(int argc, char** argv) {
+  static tokurablas_t h;
+  h.sm_count = 152;
+  cuDoubleComplex* p = (cuDoubleComplex*)4096;
+  const int st = tokura_zgeev_batched_host(&h, std::atoi(argv[1]), std::atoi(argv[2]), p, p, (char*)p, std::atoi(argv[3]));
+  for (size_t at = 0; (at = events.find("afterjoin", at)) != std::string::npos; ++at) ++waits;
+  std::printf("%d %ld %ld\n", st, solves, waits);
+}
+"""
+
 
 def linked(source, name, directory):
     """`source` with the library's object file of that translation unit."""
@@ -191,3 +228,14 @@ def test_a_failed_tuning_run_leaves_the_handle_as_it_was(tuner, kind):
     for k in range(calls):
         st, _, lanes, threads, ragged = tuner(k, kind)
         assert st == 1 and (lanes, threads, ragged) == (4, 64, 2), k
+
+
+@pytest.mark.parametrize("n,batch,chunk,in_turn", [(4, 1048576, 4096, False), (4, 30000, 0, False), (32, 65536, 8192, False),
+                                                   (33, 65536, 8192, True), (64, 65536, 0, True), (64, 30000, 2000, False)])
+def test_chunks_solved_in_turn(tmp_path, n, batch, chunk, in_turn):
+    exe = linked(HOST, "tokura_host_pipeline.cpp", tmp_path)
+    out = subprocess.run([exe, str(n), str(batch), str(chunk)], capture_output=True, text=True, timeout=60, check=True)
+    st, solves, waits = (int(v) for v in out.stdout.split())
+    assert st == 0 and solves >= 5
+    # each chunk's copy waits for the one before; in turn, its solve does too
+    assert waits == (2 if in_turn else 1) * (solves - 1)

@@ -104,11 +104,12 @@ extern "C" TOKURA_API int tokura_zgeev_batched_host(tokurablas_t* handle, int n,
   //    least 1,024 matrices each): the first solve starts after a small copy,
   //    and while the largest chunk is still arriving the earlier ones keep the
   //    GPU busy.
-  // In fixed point (tokura_handle.h: use_fixed) some thousand matrices fill the GPU, and two chunks side by side evict
-  // each other's matrices from the L2 cache: chunks of 24 matrices per SM or more are solved one after another,
-  // each beside the next one's copy, and a batch of 8 times as many is cut into 1/8, 1/4, 1/4, 1/4, 1/8, so that little
-  // is done before the first solve and after the last copy. 65,536 64 x 64 matrices: 353 ms (345 on the device) against
-  // 440-770 with two equal chunks and 500-580 with four to eight side by side.
+  // In fixed point (tokura_handle.h: use_fixed) a batch of 192 matrices per SM or more is cut into 1/8, 1/4, 1/4, 1/4, 1/8, so
+  // that little is done before the first solve and after the last copy. Above order 32, where a solve's matrices stay in the
+  // L2 cache and two solves side by side evict each other's, chunks of 24 matrices per SM or more are solved one after
+  // another, each beside the next one's copy: 65,536 64 x 64 matrices 353 ms (345 on the device) against 440-770 with
+  // two equal chunks and 500-580 with four to eight side by side. Up to order 32 they run side by side and fill each
+  // other's last waves (one after another: 30,000 of order 32 23.6 -> 27.0 ms, 1,048,576 of 4 in chunks of 4,096 5.0 -> 20.3).
   constexpr double kFastLinkGBs = 100.0;
   // One launch shape for all chunks, as for one batch.
   const tzg::PlainConfig cfg = tzg::plain_config_for(handle, n, batch_count);
@@ -145,7 +146,7 @@ extern "C" TOKURA_API int tokura_zgeev_batched_host(tokurablas_t* handle, int n,
     }
   }
   const int nchunks = (int)sizes.size();
-  bool in_turn = cfg.fixed != 0;
+  bool in_turn = cfg.fixed != 0 && n > 32;
   for (const int m : sizes) in_turn = in_turn && m >= fill;
   const int streams = nchunks < HostPipeline::kStreams ? nchunks : HostPipeline::kStreams;
   std::vector<int> cap(streams, 0);  // largest chunk each stream carries
