@@ -14,6 +14,9 @@ struct RaggedWork {
   bool square = false;  // n^2 entries apart in the workspace
   __device__ __forceinline__ bool tile(long long t, int tw, int slot, FixedTile& out) const {
     if (plan->overflow) return false;
+    // A class without matrices: two loads instead of one for each of its orders.
+    const RaggedBin &top = plan->bins[kMaxN - nhi], &low = plan->bins[kMaxN - nlo];
+    if (low.first + low.count == top.first) return false;
     for (int nb = nhi; nb >= nlo; --nb) {
       const RaggedBin& bin = plan->bins[kMaxN - nb];
       const int tiles = (bin.count + tw - 1) / tw;
