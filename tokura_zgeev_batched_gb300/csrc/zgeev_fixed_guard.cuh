@@ -26,10 +26,12 @@ constexpr int kFixedGradedIndex = 5;
 // 1e-6; k = 3, n = 3 4e-17 and 0, n = 6 4e-16 and 2e-15, n = 12 1e-13 and 2e-10; k = 10, n = 4 1e-18 and 1e-10. Relative
 // errors of dense ones, D = 1 .. 2^k: k = 6 1e-14 and 2e-14, k = 8 2e-14 and 3e-13. The scales are found in steps, all
 // indices at once, in parts of a binade; those of the matrices above span 4 binades in the third step, or never 8, and 8 in
-// the 13th at the latest. The search starts when one index's row and another's column are larger by three binades: in 1 of
-// 10,000 Gaussian matrices of order 4, 2 to 11 % of V diag V^-1 ones.
+// the 13th at the latest. The search starts when one index's row and another's column are larger by three binades, of small
+// orders by 16 / (n - 1), without which a chain of n indices does not span 8: in hardly any Gaussian matrix, 1 to 11 % of V
+// diag V^-1 ones (with three at all orders: 4,000,000 Gaussian matrices of order 2 1.86 -> 2.16 ms, 2,000,000 V diag V^-1 of
+// order 3 2.79 -> 2.89; so 1.91 and 2.81).
 constexpr int kFixedUnbalancedBits = 8;
-constexpr int kBalanceStart = 3;
+TZG_HD int balance_start(int n) { return n > 6 ? 3 : (2 * kFixedUnbalancedBits + n - 2) / (n - 1); }
 constexpr int kBalanceParts = 8;
 constexpr int kBalanceSteps = 16;
 
@@ -49,6 +51,7 @@ TZG_HD int size_exponent(unsigned size) {
 template <class Group, class First, class Top>
 TZG_HD bool left_to_fp64(const Group& G, int n, int emax, First first, Top top, int* scale) {
   bool graded = false, up = false, down = false;
+  const int start = balance_start(n);
   for (int i = G.rank; i < n; i += Group::kLanes) {
     unsigned row = 0, column = 0, diagonal = 0;
     for (int k = 0; k < n; ++k) {
@@ -64,8 +67,8 @@ TZG_HD bool left_to_fp64(const Group& G, int n, int emax, First first, Top top, 
     }
     if (row != 0 && column != 0) {
       const int d = size_exponent(row) - size_exponent(column);
-      up |= d >= kBalanceStart;
-      down |= d <= -kBalanceStart;
+      up |= d >= start;
+      down |= d <= -start;
     }
     row = diagonal > row ? diagonal : row;
     column = diagonal > column ? diagonal : column;
