@@ -86,7 +86,7 @@ def unbalanced(e):
         row, column = (off + s[:, None, :]).max(2), (off - s[:, :, None]).max(1)
         d = np.where((row > 4 * NONE) & (column > 4 * NONE), row - column - 2 * s, 0)
         if live is None:
-            start = 8 * max(3, -(-16 // (n - 1)))
+            start = 8 * (10 if n == 2 else max(3, -(-16 // (n - 1))))
             live = (d.max(1) >= start) & (d.min(1) <= -start)
         live = live & (np.abs(d).max(1) >= 4)
         s = s + np.where(live[:, None], np.sign(d) * (np.abs(d) // 2), 0)

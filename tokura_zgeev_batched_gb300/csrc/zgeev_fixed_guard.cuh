@@ -27,11 +27,11 @@ constexpr int kFixedGradedIndex = 5;
 // errors of dense ones, D = 1 .. 2^k: k = 6 1e-14 and 2e-14, k = 8 2e-14 and 3e-13. The scales are found in steps, all
 // indices at once, in parts of a binade; those of the matrices above span 4 binades in the third step, or never 8, and 8 in
 // the 13th at the latest. The search starts when one index's row and another's column are larger by three binades, of small
-// orders by 16 / (n - 1), without which a chain of n indices does not span 8: in hardly any Gaussian matrix, 1 to 11 % of V
-// diag V^-1 ones (with three at all orders: 4,000,000 Gaussian matrices of order 2 1.86 -> 2.16 ms, 2,000,000 V diag V^-1 of
+// orders by 16 / (n - 1), without which a chain of n indices does not span 8 (order 2: by 10, where two entries' digits
+// begin to differ, 9e-15 against 5e-16 at 2^12): in hardly any Gaussian matrix, 1 to 11 % of V diag V^-1 ones (with three at all orders: 4,000,000 Gaussian matrices of order 2 1.86 -> 2.16 ms, 2,000,000 V diag V^-1 of
 // order 3 2.79 -> 2.89; so 1.91 and 2.81).
 constexpr int kFixedUnbalancedBits = 8;
-TZG_HD int balance_start(int n) { return n > 6 ? 3 : (2 * kFixedUnbalancedBits + n - 2) / (n - 1); }
+TZG_HD int balance_start(int n) { return n > 6 ? 3 : n == 2 ? 10 : (2 * kFixedUnbalancedBits + n - 2) / (n - 1); }
 constexpr int kBalanceParts = 8;
 constexpr int kBalanceSteps = 16;
 
